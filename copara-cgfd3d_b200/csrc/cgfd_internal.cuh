@@ -89,6 +89,7 @@ struct StageArgs {
   int X, Y, Z;         // +1 forward / -1 backward per axis
   float h;             // steph
   float adt, bdt;      // RK4A[rk]*dt (0 for rk 3), RK4B[rk]*dt
+  float one = 1.f;     // a factor 1 that the compiler does not see
   // tW elision (the paired kernels, their traction image and sources): the
   // first stage writes no tW; the second rebuilds it from FW and the first
   // stage's output as FW + rtw * (W - FW), rtw = RK4B[0]/RK4A[0], which
@@ -198,6 +199,8 @@ struct WorkParams {
 };
 bool pair_supported(const Geom &g);
 bool pair_set_work(void *plan, const WorkParams &wp);
+// per model: StageArgs::plain_interior (rebuilds the work lists on a change)
+bool pair_set_plain(void *plan, const char *plain);
 // test hook (cgfd_test_withhold_copy): every wait of the plan's kernels gives
 // up after wait_s, and with withhold >= 0 the velocity part's CTA 0 does not
 // issue the halo copy of entry `withhold` of its first item; withhold < 0
@@ -207,19 +210,19 @@ WorkParams pair_get_work(const void *plan);
 void *pair_create_plan(const Geom &g, int elem, void *const sets[4], const float *media,
                        const float *metric, float *const aux[3]);
 void pair_destroy_plan(void *plan);
-// a second stream and two events (cudaStream_t / cudaEvent_t) for work
-// that may run beside the stage kernels
+// side streams (cudaStream_t) and the events (cudaEvent_t) that fork them
+// from the solver's stream and join them to it, for launches of one stage
+// that may run beside one another
 struct SideStream {
-  void *stream, *fork, *join;
-  void *stream2, *fork2, *join2;  // the stress part beside the velocity part
+  static constexpr int N = 3;
+  void *stream[N], *join[N], *fork;
 };
 // the paired kernels run with a.tw_skip set (tW elision); with side, the
-// traction image runs on side->stream and the stress part on side->stream2,
-// beside the velocity part (the three read only the stage input and write
-// disjoint components)
+// launches of a stage run beside one another on its streams (they read only
+// the stage input and write disjoint values)
 void launch_stage_pair(const void *plan, const StageArgs &a, int in_set, int *err, void *stream,
                        const SideStream *side = nullptr);
-int pair_plan_info(const void *plan, int *zchunk, int *grid_vel, int *grid_str);
+int pair_plan_info(const void *plan, int *zchunk, int *grid_general, int *grid_lean);
 // A batch of models (one storage type) in one persistent launch per stage
 // part: per-model buffers as n x 4 sets, n media, n metrics, n x 3
 // auxiliaries.

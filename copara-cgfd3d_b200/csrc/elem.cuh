@@ -31,11 +31,23 @@ template <> struct Elem<__half> {
   static constexpr int kind = ELEM_F16;
   __device__ __forceinline__ static float ld(const __half *p) { return __half2float(*p); }
   __device__ __forceinline__ static void st(__half *p, float v) { *p = __float2half_rn(v); }
+  // a pair as its 32 bits
+  __device__ __forceinline__ static float2 widen(unsigned u) {
+    float2 r;
+    asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %2;\n cvt.f32.f16 %0, l;\n cvt.f32.f16 %1, h;\n}"
+        : "=f"(r.x), "=f"(r.y) : "r"(u));
+    return r;
+  }
+  __device__ __forceinline__ static unsigned narrow(float2 v) {
+    unsigned u;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(u) : "f"(v.y), "f"(v.x));
+    return u;
+  }
   __device__ __forceinline__ static float2 ld2(const __half *p) {
-    return __half22float2(*reinterpret_cast<const __half2 *>(p));
+    return widen(*reinterpret_cast<const unsigned *>(p));
   }
   __device__ __forceinline__ static void st2(__half *p, float2 v) {
-    *reinterpret_cast<__half2 *>(p) = __float22half2_rn(v);
+    *reinterpret_cast<unsigned *>(p) = narrow(v);
   }
 };
 
@@ -47,11 +59,19 @@ template <> struct Elem<__nv_bfloat16> {
   __device__ __forceinline__ static void st(__nv_bfloat16 *p, float v) {
     *p = __float2bfloat16_rn(v);
   }
+  __device__ __forceinline__ static float2 widen(unsigned u) {  // BF16 is FP32's upper half
+    return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+  }
+  __device__ __forceinline__ static unsigned narrow(float2 v) {
+    unsigned u;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(u) : "f"(v.y), "f"(v.x));
+    return u;
+  }
   __device__ __forceinline__ static float2 ld2(const __nv_bfloat16 *p) {
-    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(p));
+    return widen(*reinterpret_cast<const unsigned *>(p));
   }
   __device__ __forceinline__ static void st2(__nv_bfloat16 *p, float2 v) {
-    *reinterpret_cast<__nv_bfloat162 *>(p) = __float22bfloat162_rn(v);
+    *reinterpret_cast<unsigned *>(p) = narrow(v);
   }
 };
 

@@ -1,0 +1,6 @@
+// pair_f0l.cu -- the paired stage kernels over the lean items,
+// RK stage kind 0 (first stage), FP32 storage, for the 8 stencil directions,
+// single-model and batched.
+#include "stage_pair_impl.cuh"
+
+cgfd::pair::Entry cgfd::pair::entry_f0l() { return make_entry<float, 0, LEAN_BOTH>(); }

@@ -1,0 +1,6 @@
+// pair_f1v.cu -- the paired stage kernels over the velocity part of the general items,
+// RK stage kind 1 (inner stages), FP32 storage, for the 8 stencil directions,
+// single-model and batched.
+#include "stage_pair_impl.cuh"
+
+cgfd::pair::Entry cgfd::pair::entry_f1v() { return make_entry<float, 1, GEN_VEL>(); }

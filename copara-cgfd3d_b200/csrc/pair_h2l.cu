@@ -1,0 +1,6 @@
+// pair_h2l.cu -- the paired stage kernels over the lean items,
+// RK stage kind 2 (final stage), FP16 storage, for the 8 stencil directions,
+// single-model and batched.
+#include "stage_pair_impl.cuh"
+
+cgfd::pair::Entry cgfd::pair::entry_h2l() { return make_entry<__half, 2, LEAN_BOTH>(); }

@@ -373,8 +373,7 @@ struct cgfd_solver {
   cgfd_desc d{};
   Geom g{};
   cudaStream_t st = nullptr;
-  // traction image and stress part beside the velocity part
-  SideStream side{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  SideStream side{};  // the launches of a stage beside one another
   // host-to-device upload staging: the copy events of the two pinned chunks
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
   std::string err;
@@ -525,12 +524,11 @@ void free_all(cgfd_solver *h) {
   if (h->st) cudaStreamDestroy(h->st);
   for (int q = 0; q < 2; ++q)
     if (h->pin_ev[q]) cudaEventDestroy(h->pin_ev[q]);
-  if (h->side.stream) cudaStreamDestroy((cudaStream_t)h->side.stream);
   if (h->side.fork) cudaEventDestroy((cudaEvent_t)h->side.fork);
-  if (h->side.join) cudaEventDestroy((cudaEvent_t)h->side.join);
-  if (h->side.stream2) cudaStreamDestroy((cudaStream_t)h->side.stream2);
-  if (h->side.fork2) cudaEventDestroy((cudaEvent_t)h->side.fork2);
-  if (h->side.join2) cudaEventDestroy((cudaEvent_t)h->side.join2);
+  for (int q = 0; q < SideStream::N; ++q) {
+    if (h->side.stream[q]) cudaStreamDestroy((cudaStream_t)h->side.stream[q]);
+    if (h->side.join[q]) cudaEventDestroy((cudaEvent_t)h->side.join[q]);
+  }
 }
 
 long ref_n(const cgfd_solver *h) {
@@ -1018,22 +1016,18 @@ int cgfd_create(const cgfd_desc *d, cgfd_solver **out) {
     if (e == cudaSuccess) e = cudaMalloc(&h->d_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(h->d_err, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
-    cudaStream_t s2 = nullptr;
-    cudaEvent_t e1 = nullptr, e2 = nullptr;
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking);
-    h->side.stream = s2;
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&e1, cudaEventDisableTiming);
-    h->side.fork = e1;
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&e2, cudaEventDisableTiming);
-    h->side.join = e2;
-    cudaStream_t s3 = nullptr;
-    cudaEvent_t e3 = nullptr, e4 = nullptr;
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s3, cudaStreamNonBlocking);
-    h->side.stream2 = s3;
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&e3, cudaEventDisableTiming);
-    h->side.fork2 = e3;
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&e4, cudaEventDisableTiming);
-    h->side.join2 = e4;
+    auto event = [&](void **out) {
+      cudaEvent_t ev = nullptr;
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+      *out = ev;
+    };
+    event(&h->side.fork);
+    for (int q = 0; q < SideStream::N; ++q) {
+      cudaStream_t s2 = nullptr;
+      if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking);
+      h->side.stream[q] = s2;
+      event(&h->side.join[q]);
+    }
     if (e != cudaSuccess) st = cuda_fail(nullptr, e, "setup");
   }
   if (st) {
@@ -1644,6 +1638,10 @@ int cgfd_prepare(cgfd_solver *h) {
     int st2 = apply_scales(h, e);
     if (st2) return st2;
   }
+  if (h->d.kernel == CGFD_KERNEL_FUSED) {
+    const char plain = h->plain_interior;
+    if (!pair_set_plain(h->plan, &plain)) return cuda_fail(h, cudaErrorUnknown, "work list");
+  }
   h->prepared = true;
   int st = build_graphs(h);
   if (st) return st;
@@ -2208,6 +2206,10 @@ static int batch_build(cgfd_batch *b) {
                                      aux.data(), b->elem);
     if (!b->plan) return batch_fail(b, CGFD_ERR_CUDA, "batch plan (tensor maps or work list)");
   }
+  std::vector<char> plain(n);
+  for (int i = 0; i < n; ++i) plain[i] = b->m[i]->plain_interior;
+  if (!pair_set_plain(b->plan, plain.data()))
+    return batch_fail(b, CGFD_ERR_CUDA, "batch work list");
   if (!pair_batch_set_args(b->plan, args.data()))
     return batch_fail(b, CGFD_ERR_CUDA, "batch stage arguments");
   if (!b->d_src) BCK(b, cudaMalloc(&b->d_src, src.size() * sizeof(SourceArgs)));

@@ -1,7 +1,7 @@
 // stage_pair.cu -- host side of the paired z-marching stage kernels: TMA
 // tensor maps, launch plan (persistent grid, z-chunk length) and dispatch.
 // The kernels themselves are in stage_pair_impl.cuh, instantiated by
-// pair_{v,s}{0,1,2}.cu.
+// pair_*.cu.
 #include "stage_pair_impl.cuh"
 
 #include <algorithm>
@@ -76,15 +76,23 @@ bool pair_supported(const Geom &g) {
 namespace pair {
 namespace {
 
+// entry points by storage type (ELEM_*), RK stage kind and launch
+const Entry &entry(int elem, int kind, int list) {
+#define CGFD_ENTRIES(E)                                  \
+  {{entry_##E##0v(), entry_##E##0s(), entry_##E##0l()},  \
+   {entry_##E##1v(), entry_##E##1s(), entry_##E##1l()},  \
+   {entry_##E##2v(), entry_##E##2s(), entry_##E##2l()}}
+  static const Entry e[3][3][NLIST] = {CGFD_ENTRIES(f), CGFD_ENTRIES(h), CGFD_ENTRIES(b)};
+#undef CGFD_ENTRIES
+  return e[elem][kind][list];
+}
+
 void set_all_attrs() {
   static bool done = false;
   if (done) return;
-  attrs_fv0(); attrs_fv1(); attrs_fv2(); attrs_fs0(); attrs_fs1(); attrs_fs2();
-  attrs_hv0(); attrs_hv1(); attrs_hv2(); attrs_hs0(); attrs_hs1(); attrs_hs2();
-  attrs_bv0(); attrs_bv1(); attrs_bv2(); attrs_bs0(); attrs_bs1(); attrs_bs2();
-  attrs_fv0_b(); attrs_fv1_b(); attrs_fv2_b(); attrs_fs0_b(); attrs_fs1_b(); attrs_fs2_b();
-  attrs_hv0_b(); attrs_hv1_b(); attrs_hv2_b(); attrs_hs0_b(); attrs_hs1_b(); attrs_hs2_b();
-  attrs_bv0_b(); attrs_bv1_b(); attrs_bv2_b(); attrs_bs0_b(); attrs_bs1_b(); attrs_bs2_b();
+  for (int elem = 0; elem < 3; ++elem)
+    for (int kind = 0; kind < 3; ++kind)
+      for (int list = 0; list < NLIST; ++list) entry(elem, kind, list).attrs();
   done = true;
 }
 
@@ -142,102 +150,131 @@ void stage_maps(const ModelMaps &pl, int rk, int in_set, bool rebuild, bool tw_d
   }
 }
 
-// x origin of the tile grid (tiles start at i = t * CX - offset).  The
-// stage kernels' time follows the number of tile-planes, and a tile that
-// touches an x layer runs the slower boundary path for all its columns.
-// Candidates 0 and 32 keep every tile row of the field, media and metric
-// boxes on a 128-byte boundary (the internal x origin XO is 32); 32 is taken
-// when it needs no more tile columns and puts fewer valid columns into tiles
-// that touch an x layer (on the 400-wide hill with 20-cell layers: 80
-// instead of 144 columns).
-int tile_x_offset(const Geom &g) {
-  auto ntx = [&](int o) { return (g.ni + o + CX - 1) / CX; };
-  auto boundary_cols = [&](int o) {
-    int n = 0;
-    for (int t = 0; t < ntx(o); ++t) {
-      const int i0 = t * CX - o, a = std::max(i0, 0), b = std::min(i0 + CX, g.ni);
-      if (a < g.nabs[0] || b > g.ni - g.nabs[1]) n += b - a;
-    }
-    return n;
-  };
-  return (ntx(32) == ntx(0) && boundary_cols(32) < boundary_cols(0)) ? 32 : 0;
+// Tile origins along one axis of n cells with layers of lo and hi cells:
+// tiles of `size` cells that start at `first`, tiles inside the layers' inner
+// faces marked interior.
+struct Tile {
+  int at;
+  bool interior;
+};
+// x: origins at multiples of CX from 0, which keeps every tile row of the
+// field, media and metric boxes on a 128-byte boundary
+std::vector<Tile> x_tiles(const Geom &g) {
+  std::vector<Tile> t;
+  for (int i = 0; i < g.ni; i += CX)
+    t.push_back({i, i >= g.nabs[0] && i + CX <= g.ni - g.nabs[1]});
+  return t;
+}
+// y: the interior tiles start at the low layer's inner face (its own tiles
+// lie before them, the first one partly left of the grid when the layer is
+// no multiple of TY), so that layers of any width cost no more boundary tiles
+// than they fill
+std::vector<Tile> y_tiles(const Geom &g) {
+  std::vector<Tile> t;
+  const int lo = g.nabs[2], nin = (g.nj - lo - g.nabs[3]) / TY;
+  for (int j = lo - (lo + TY - 1) / TY * TY; j < g.nj; j += TY)
+    t.push_back({j, j >= lo && j < lo + nin * TY});
+  return t;
 }
 
-// Work items of one or more models (tile x z-chunk): the bottom PML layer is
-// a z-chunk of its own (when it has >= 8 planes), the rest is cut into pieces
-// of about len planes (>= MIN_CHUNK; every chunk has >= 4 planes, which the
-// kernel's initial issue of four entries relies on).  Order: the most
-// expensive first (estimated cost: planes x sum over the tile's valid
-// columns of (1 + pml_weight x number of PML directions)), so the cheap
-// items fill the tail; equal costs keep the (model, z-chunk, tile) order, so
-// neighbouring tiles of a class run together and share halo rows in L2.
-std::vector<int4> build_items(const std::vector<Geom> &gs, int G, const WorkParams &wp,
-                              int *zchunk) {
-  // target chunk length: enough items (items_per_cta per resident CTA) over
-  // all models' tile columns
-  double colplanes = 0;
-  for (const Geom &g : gs)
-    colplanes += (double)((g.ni + CX - 1) / CX) * ((g.nj + TY - 1) / TY) * g.nk;
-  const double target = (double)wp.items_per_cta * G;
+// Work items of one or more models, in two lists: lean items (no PML cell, no
+// cell outside the grid; `plain` models only) and general ones.  Item: tile
+// origin, z range, 2 * model + part.  The bottom PML layer is a z-chunk of
+// its own (in general columns when it has >= 8 planes), the rest is cut into
+// pieces.  Order: the most expensive first (estimated cost: planes x sum over
+// the tile's valid columns of (1 + pml_weight x number of PML directions)), so
+// the cheap items fill the tail; equal costs keep the (model, z-chunk, tile)
+// order, so neighbouring tiles of a class run together and share halo rows in
+// L2, and the two parts of a tile follow one another.
+std::vector<int4> build_items(const std::vector<Geom> &gs, const std::vector<char> &plain,
+                              bool lean, int G, const WorkParams &wp, int *zchunk) {
   struct It { int4 v; double cost; };
-  std::vector<It> items;
+  struct Col { int i0, j0, z0, z1, mdl; double w; bool cut; };
+  std::vector<Col> cols;  // columns with their z range, to be cut into pieces
+  double planes = 0;
   for (size_t mdl = 0; mdl < gs.size(); ++mdl) {
     const Geom &g = gs[mdl];
-    const int xoff = tile_x_offset(g);
-    const int ntx = (g.ni + xoff + CX - 1) / CX, nty = (g.nj + TY - 1) / TY;
-    const int ntiles = ntx * nty;
-    std::vector<int> zb{LFD};
     const int zlo = LFD + g.nabs[4], ztop = g.nk + LFD;
-    if (g.nabs[4] >= 8 && ztop - zlo >= 8) zb.push_back(zlo);
-    const int zr = zb.back(), rest = ztop - zr;
-    int pieces = 1;
-    if (gs.size() == 1) {
-      while ((long)ntiles * ((long)zb.size() - 1 + pieces) < (long)target &&
-             rest / (pieces + 1) >= wp.min_chunk)
-        ++pieces;
-    } else {
-      const double len = colplanes / target > wp.min_chunk ? colplanes / target : wp.min_chunk;
-      pieces = (int)(rest / len + 0.5);
-      if (pieces < 1) pieces = 1;
-      while (pieces > 1 && rest / pieces < 4) --pieces;
-    }
-    for (int q = 1; q <= pieces; ++q) zb.push_back(zr + (int)((long)rest * q / pieces));
-    if (zchunk && mdl == 0) *zchunk = (rest + pieces - 1) / pieces;
-    for (size_t c = 0; c + 1 < zb.size(); ++c) {
-      if (zb[c + 1] - zb[c] < 4) return {};
-      const bool zp = zb[c] < zlo;
-      for (int t = 0; t < ntiles; ++t) {
-        const int i0 = (t % ntx) * CX - xoff, j0 = (t / ntx) * TY;
-        double w = 0;
-        for (int j = j0; j < j0 + TY && j < g.nj; ++j) {
-          const bool yp = j < g.nabs[2] || j >= g.nj - g.nabs[3];
-          for (int i = std::max(i0, 0); i < i0 + CX && i < g.ni; ++i) {
-            const bool xp = i < g.nabs[0] || i >= g.ni - g.nabs[1];
-            w += 1 + wp.pml_weight * ((xp ? 1 : 0) + (yp ? 1 : 0) + (zp ? 1 : 0));
+    const bool split = plain[mdl] && ztop - zlo >= 8;  // lean columns exist
+    for (const Tile &ty : y_tiles(g))
+      for (const Tile &tx : x_tiles(g)) {
+        const bool in = split && tx.interior && ty.interior;
+        if (lean && !in) continue;
+        auto add = [&](int z0, int z1, bool cut) {
+          if (z0 >= z1) return;
+          double w = 0;
+          for (int j = std::max(ty.at, 0); j < ty.at + TY && j < g.nj; ++j) {
+            const bool yp = j < g.nabs[2] || j >= g.nj - g.nabs[3];
+            for (int i = tx.at; i < tx.at + CX && i < g.ni; ++i) {
+              const bool xp = i < g.nabs[0] || i >= g.ni - g.nabs[1];
+              w += 1 + wp.pml_weight * ((xp ? 1 : 0) + (yp ? 1 : 0) + (z0 < zlo ? 1 : 0));
+            }
           }
+          cols.push_back({tx.at, ty.at, z0, z1, (int)mdl, w, cut});
+          planes += z1 - z0;
+        };
+        if (lean) {
+          add(zlo, ztop, true);
+        } else if (in) {
+          add(LFD, zlo, true);
+        } else if (g.nabs[4] >= 8 && ztop - zlo >= 8) {
+          add(LFD, zlo, true);
+          add(zlo, ztop, true);
+        } else {
+          add(LFD, ztop, true);
         }
-        items.push_back({make_int4(i0, j0, zb[c] | (zb[c + 1] << 16), (int)mdl),
-                         w * (zb[c + 1] - zb[c])});
       }
+  }
+  if (cols.empty()) return {};
+  // chunk length: about items_per_cta items per resident CTA, at
+  // least min_chunk planes; but where that leaves resident CTAs without an
+  // item, chunks down to MIN_LEN planes
+  constexpr int MIN_LEN = 4;
+  const int parts = lean ? 2 : 1;
+  const double fill = parts * planes / G;
+  double len = std::max(fill / wp.items_per_cta, (double)wp.min_chunk);
+  if (fill < len) len = std::max(fill, (double)MIN_LEN);
+  std::vector<It> items;
+  for (const Col &c : cols) {
+    const int n = c.z1 - c.z0;
+    int pieces = std::max(1, (int)(n / len + 0.5));
+    while (pieces > 1 && n / pieces < MIN_LEN) --pieces;
+    if (zchunk && items.empty()) *zchunk = (n + pieces - 1) / pieces;
+    for (int q = 0; q < pieces; ++q) {
+      const int a0 = c.z0 + (int)((long)n * q / pieces);
+      const int a1 = c.z0 + (int)((long)n * (q + 1) / pieces);
+      items.push_back({make_int4(c.i0, c.j0, a0 | (a1 << 16), c.mdl), c.w * (a1 - a0)});
     }
   }
-  std::stable_sort(items.begin(), items.end(),
-                   [](const It &x, const It &y) { return x.cost > y.cost; });
+  // z-chunks of a class together: columns were cut one by one
+  std::stable_sort(items.begin(), items.end(), [](const It &x, const It &y) {
+    if (x.cost != y.cost) return x.cost > y.cost;
+    if (x.v.w != y.v.w) return x.v.w < y.v.w;
+    return (x.v.z & 0xffff) < (y.v.z & 0xffff);
+  });
   std::vector<int4> hv;
-  hv.reserve(items.size());
-  // guided end: the last G items (the cheapest) become short chunks, ordered
-  // piece by piece (the first piece of every cut item, then the second...)
-  // so that CTAs running together stay on neighbouring columns
+  hv.reserve(2 * items.size());
+  auto push = [&](int4 v) {
+    v.w *= 2;
+    hv.push_back(v);  // PART_VEL
+    if (!lean) return;
+    v.w += 1;
+    hv.push_back(v);  // PART_STR
+  };
+  // guided end: the last items (the cheapest, one per resident CTA) become
+  // short chunks, ordered piece by piece (the first piece of every cut item,
+  // then the second...) so that CTAs running together stay on neighbouring
+  // columns
   size_t ncut = 0;
   if (wp.tail_chunk >= 4) {
-    while (ncut < (size_t)G && ncut < items.size()) {
+    while (parts * ncut < (size_t)G && ncut < items.size()) {
       const int4 v = items[items.size() - 1 - ncut].v;
       if ((v.z >> 16) - (v.z & 0xffff) < 2 * wp.tail_chunk) break;
       ++ncut;
     }
   }
   const size_t keep = items.size() - ncut;
-  for (size_t q = 0; q < keep; ++q) hv.push_back(items[q].v);
+  for (size_t q = 0; q < keep; ++q) push(items[q].v);
   std::vector<std::vector<int4>> pieces(ncut);
   size_t maxp = 0;
   for (size_t q = 0; q < ncut; ++q) {
@@ -252,43 +289,40 @@ std::vector<int4> build_items(const std::vector<Geom> &gs, int G, const WorkPara
   }
   for (size_t t = 0; t < maxp; ++t)
     for (size_t q = 0; q < ncut; ++q)
-      if (t < pieces[q].size()) hv.push_back(pieces[q][t]);
+      if (t < pieces[q].size()) push(pieces[q][t]);
   return hv;
 }
 
-// uploads a work list into the plan (replacing an earlier one)
-bool upload_items(Plan *pl, const std::vector<int4> &hv, int rv, int rs) {
+// uploads the two work lists into the plan (replacing earlier ones)
+bool upload_items(Plan *pl, const std::vector<int4> (&hv)[2],
+                  const int (&G)[NLIST]) {
   Work &wk = pl->wk;
-  if (hv.empty()) return false;
-  cudaFree((void *)wk.items);
-  wk.items = nullptr;
-  int4 *d_items = nullptr;
-  if (cudaMalloc(&d_items, hv.size() * sizeof(int4)) != cudaSuccess ||
-      cudaMemcpy(d_items, hv.data(), hv.size() * sizeof(int4), cudaMemcpyHostToDevice) !=
-          cudaSuccess) {
-    cudaFree(d_items);
-    return false;
+  if (hv[0].empty() && hv[1].empty()) return false;
+  for (int l = 0; l < 2; ++l) {
+    cudaFree((void *)wk.items[l]);
+    wk.items[l] = nullptr;
+    wk.nitems[l] = (int)hv[l].size();
+    if (hv[l].empty()) continue;
+    int4 *d_items = nullptr;
+    if (cudaMalloc(&d_items, hv[l].size() * sizeof(int4)) != cudaSuccess ||
+        cudaMemcpy(d_items, hv[l].data(), hv[l].size() * sizeof(int4), cudaMemcpyHostToDevice) !=
+            cudaSuccess) {
+      cudaFree(d_items);
+      wk.nitems[l] = 0;
+      return false;
+    }
+    wk.items[l] = d_items;
+  }
+  for (int q = 0; q < NLIST; ++q) {
+    const int n = wk.nitems[q == LEAN_BOTH];
+    pl->grid[q] = n < G[q] ? n : G[q];
   }
   if (!wk.counter) {
-    if (cudaMalloc(&wk.counter, 2 * sizeof(int)) != cudaSuccess ||
-        cudaMemset(wk.counter, 0, 2 * sizeof(int)) != cudaSuccess)
+    if (cudaMalloc(&wk.counter, 2 * NLIST * sizeof(int)) != cudaSuccess ||
+        cudaMemset(wk.counter, 0, 2 * NLIST * sizeof(int)) != cudaSuccess)
       return false;
   }
-  wk.items = d_items;
-  wk.nitems = (int)hv.size();
-  pl->grid[0] = wk.nitems < rv ? wk.nitems : rv;
-  pl->grid[1] = wk.nitems < rs ? wk.nitems : rs;
   return true;
-}
-
-void resident(int elem, bool batch, int *rv, int *rs) {
-  if (batch) {
-    *rv = elem == ELEM_F16 ? resident_hv_b() : elem == ELEM_BF16 ? resident_bv_b() : resident_fv_b();
-    *rs = elem == ELEM_F16 ? resident_hs_b() : elem == ELEM_BF16 ? resident_bs_b() : resident_fs_b();
-  } else {
-    *rv = elem == ELEM_F16 ? resident_hv() : elem == ELEM_BF16 ? resident_bv() : resident_fv();
-    *rs = elem == ELEM_F16 ? resident_hs() : elem == ELEM_BF16 ? resident_bs() : resident_fs();
-  }
 }
 
 }  // namespace
@@ -301,6 +335,7 @@ void *pair_create_plan(const Geom &g, int elem, void *const sets[4], const float
   if (!pl) return nullptr;
   pl->elem = elem;
   pl->geoms.push_back(g);
+  pl->plain.assign(1, 1);
   pl->mm.resize(1);
   if (!model_maps(&pl->mm[0], pl->wk.has_aux, g, elem, sets, media, metric, aux) ||
       !pair_set_work(pl, WorkParams{})) {
@@ -316,13 +351,23 @@ WorkParams pair_get_work(const void *plan) {
 
 bool pair_set_work(void *plan, const WorkParams &wp) {
   Plan *pl = reinterpret_cast<Plan *>(plan);
-  int rv = 0, rs = 0;
-  resident(pl->elem, pl->nmodels > 0, &rv, &rs);
-  const int G = rv < rs ? rv : rs;
-  std::vector<int4> hv = build_items(pl->geoms, G, wp, &pl->zchunk);
-  if (!upload_items(pl, hv, rv, rs)) return false;
+  std::vector<int4> hv[2];
+  int G[NLIST];
+  for (int q = 0; q < NLIST; ++q) G[q] = entry(pl->elem, 1, q).resident[pl->nmodels > 0]();
+  for (int l = 0; l < 2; ++l)
+    hv[l] = build_items(pl->geoms, pl->plain, l != 0,
+                        l ? G[LEAN_BOTH] : std::min(G[GEN_VEL], G[GEN_STR]), wp, &pl->zchunk);
+  if (!upload_items(pl, hv, G)) return false;
   pl->params = wp;
   return true;
+}
+
+bool pair_set_plain(void *plan, const char *plain) {
+  Plan *pl = reinterpret_cast<Plan *>(plan);
+  const std::vector<char> v(plain, plain + pl->geoms.size());
+  if (v == pl->plain) return true;
+  pl->plain = v;
+  return pair_set_work(plan, pl->params);
 }
 
 bool pair_set_wait_test(void *plan, double wait_s, int withhold) {
@@ -336,7 +381,7 @@ bool pair_set_wait_test(void *plan, double wait_s, int withhold) {
 void pair_destroy_plan(void *plan) {
   Plan *pl = reinterpret_cast<Plan *>(plan);
   if (!pl) return;
-  cudaFree((void *)pl->wk.items);
+  for (const int4 *p : pl->wk.items) cudaFree((void *)p);
   cudaFree(pl->wk.counter);
   cudaFree(pl->d_bargs);
   cudaFree(pl->d_bmaps);
@@ -348,42 +393,28 @@ void launch_stage_pair(const void *plan, const StageArgs &a, int in_set, int *er
   const Plan &pl = *reinterpret_cast<const Plan *>(plan);
   cudaStream_t s = (cudaStream_t)stream;
   const int kind = a.rk == 0 ? 0 : (a.rk < 3 ? 1 : 2);
-  Maps mv, ms;
-  stage_maps(pl.mm[0], a.rk, in_set, a.tw_skip && a.rk == 1, pl.elem != ELEM_F32, mv, ms);
-  // the traction image needs only the stage input and writes what the two
-  // parts neither write nor use (the top three layers' V, their tW and x/y
-  // auxiliaries): with a side stream it runs beside them, joined at the end
+  Maps m[2];
+  stage_maps(pl.mm[0], a.rk, in_set, a.tw_skip && a.rk == 1, pl.elem != ELEM_F32, m[0], m[1]);
+  // the parts of the general items, the lean items and the traction image (the
+  // top three layers' V, their tW and x/y auxiliaries) need only the stage
+  // input and write disjoint values: with side streams they run beside one
+  // another
+  cudaStream_t ls[NLIST] = {s, s, s};
   if (side) {
     cudaEventRecord((cudaEvent_t)side->fork, s);
-    cudaStreamWaitEvent((cudaStream_t)side->stream, (cudaEvent_t)side->fork, 0);
-    launch_timg(a, side->stream);
-    cudaEventRecord((cudaEvent_t)side->join, (cudaStream_t)side->stream);
+    for (int q = 0; q < SideStream::N; ++q)
+      cudaStreamWaitEvent((cudaStream_t)side->stream[q], (cudaEvent_t)side->fork, 0);
+    if (pl.grid[GEN_STR] > 0) ls[GEN_STR] = (cudaStream_t)side->stream[1];
+    if (pl.grid[GEN_VEL] > 0) ls[LEAN_BOTH] = (cudaStream_t)side->stream[2];
   }
-  // both parts' item counters restart at zero
-  cudaMemsetAsync(pl.wk.counter, 0, 2 * sizeof(int), s);
-  // the stress part needs the stage input's velocities, not the velocity
-  // part's output, and writes other components: with a second side stream
-  // its CTAs take the SMs as the velocity part's drain
-  cudaStream_t s2 = s;
-  if (side && side->stream2) {
-    s2 = (cudaStream_t)side->stream2;
-    cudaEventRecord((cudaEvent_t)side->fork2, s);
-    cudaStreamWaitEvent(s2, (cudaEvent_t)side->fork2, 0);
-  }
-  typedef void (*LaunchFn)(const Plan &, const Maps &, const StageArgs &, int *, cudaStream_t);
-  static const LaunchFn fns[3][2][3] = {
-      {{launch_fv0, launch_fv1, launch_fv2}, {launch_fs0, launch_fs1, launch_fs2}},
-      {{launch_hv0, launch_hv1, launch_hv2}, {launch_hs0, launch_hs1, launch_hs2}},
-      {{launch_bv0, launch_bv1, launch_bv2}, {launch_bs0, launch_bs1, launch_bs2}}};
-  const int e = pl.elem == ELEM_F16 ? 1 : pl.elem == ELEM_BF16 ? 2 : 0;
-  fns[e][0][kind](pl, mv, a, err, s);
-  fns[e][1][kind](pl, ms, a, err, s2);
-  if (s2 != s) {
-    cudaEventRecord((cudaEvent_t)side->join2, s2);
-    cudaStreamWaitEvent(s, (cudaEvent_t)side->join2, 0);
-  }
-  if (side) cudaStreamWaitEvent(s, (cudaEvent_t)side->join, 0);
-  else launch_timg(a, s);
+  for (int q : {GEN_STR, GEN_VEL, LEAN_BOTH})
+    if (pl.grid[q] > 0) entry(pl.elem, kind, q).launch[0](pl, m, a, pl.wk, err, ls[q]);
+  launch_timg(a, side ? side->stream[0] : stream);
+  if (side)
+    for (int q = 0; q < SideStream::N; ++q) {
+      cudaEventRecord((cudaEvent_t)side->join[q], (cudaStream_t)side->stream[q]);
+      cudaStreamWaitEvent(s, (cudaEvent_t)side->join[q], 0);
+    }
 }
 
 // ---------------------------- batched models ------------------------------
@@ -396,6 +427,8 @@ void *pair_create_batch_plan(int n, const Geom *gs, void *const *sets, const flo
   pl->elem = elem;
   pl->nmodels = n;
   pl->geoms.assign(gs, gs + n);
+  pl->plain.assign(n, 1);
+  pl->wk.nmodels = n;
   pl->mm.resize(n);
   bool ok = true;
   for (int i = 0; i < n && ok; ++i) {
@@ -434,35 +467,26 @@ void launch_stage_pair_batch(const void *plan, int pattern, const StageArgs &rep
   const Plan &pl = *reinterpret_cast<const Plan *>(plan);
   cudaStream_t s = (cudaStream_t)stream;
   const int rk = rep.rk, kind = rk == 0 ? 0 : (rk < 3 ? 1 : 2), n = pl.nmodels;
-  Work wv = pl.wk, ws = pl.wk;
-  wv.bargs = ws.bargs = pl.d_bargs + (size_t)(pattern * 4 + rk) * n;
-  wv.bmaps = pl.d_bmaps + (size_t)(rk * 2) * n;
-  ws.bmaps = pl.d_bmaps + (size_t)(rk * 2 + 1) * n;
-  typedef void (*LaunchFn)(const Plan &, const StageArgs &, const Work &, int *, cudaStream_t);
-  static const LaunchFn fv[3][3] = {{launch_fv0_b, launch_fv1_b, launch_fv2_b},
-                                    {launch_hv0_b, launch_hv1_b, launch_hv2_b},
-                                    {launch_bv0_b, launch_bv1_b, launch_bv2_b}};
-  static const LaunchFn fs[3][3] = {{launch_fs0_b, launch_fs1_b, launch_fs2_b},
-                                    {launch_hs0_b, launch_hs1_b, launch_hs2_b},
-                                    {launch_bs0_b, launch_bs1_b, launch_bs2_b}};
-  const int e = pl.elem == ELEM_F16 ? 1 : pl.elem == ELEM_BF16 ? 2 : 0;
-  cudaMemsetAsync(pl.wk.counter, 0, 2 * sizeof(int), s);
-  fv[e][kind](pl, rep, wv, err, s);
-  fs[e][kind](pl, rep, ws, err, s);
+  Work wk = pl.wk;
+  wk.bargs = pl.d_bargs + (size_t)(pattern * 4 + rk) * n;
+  wk.bmaps = pl.d_bmaps + (size_t)(rk * 2) * n;
+  const Maps none[2] = {};
+  for (int q : {GEN_STR, GEN_VEL, LEAN_BOTH})
+    if (pl.grid[q] > 0) entry(pl.elem, kind, q).launch[1](pl, none, rep, wk, err, s);
   int mi = 0, mj = 0;
   for (const Geom &g : pl.geoms) {
     mi = g.ni > mi ? g.ni : mi;
     mj = g.nj > mj ? g.nj : mj;
   }
-  launch_timg_batch(wv.bargs, n, mi, mj, pl.elem, s);
+  launch_timg_batch(wk.bargs, n, mi, mj, pl.elem, s);
 }
 
-int pair_plan_info(const void *plan, int *zchunk, int *grid_vel, int *grid_str) {
+int pair_plan_info(const void *plan, int *zchunk, int *grid_general, int *grid_lean) {
   const Plan &pl = *reinterpret_cast<const Plan *>(plan);
   if (zchunk) *zchunk = pl.zchunk;
-  if (grid_vel) *grid_vel = pl.grid[0];
-  if (grid_str) *grid_str = pl.grid[1];
-  return pl.wk.nitems;
+  if (grid_general) *grid_general = pl.grid[GEN_VEL];
+  if (grid_lean) *grid_lean = pl.grid[LEAN_BOTH];
+  return pl.wk.nitems[0] + pl.wk.nitems[1];
 }
 
 }  // namespace cgfd

@@ -1,12 +1,25 @@
 // stage_pair_impl.cuh -- z-marching RK stage kernels for sm_100a with two
 // x-adjacent cells per thread (templates; instantiated by pair_*.cu).
 //
-// One RK stage is two kernels, split along the velocity-stress structure of
-// the equations: the velocity part differentiates only the six stresses and
-// the stress part only the three velocities.  A CTA of 32 x 4 threads owns a
-// tile of 64 x 4 (x, y) columns, each thread the cell pair (2t, 2t+1) of its
-// row, and marches through a chunk of z-planes; a persistent grid of CTAs
-// (two per SM) walks the (tile, z-chunk) items.
+// One RK stage is split along the velocity-stress structure of the equations:
+// the velocity part differentiates only the six stresses and the stress part
+// only the three velocities.  A CTA of 16 x 8 threads owns a tile of 32 x 8
+// (x, y) columns, each thread the cell pair (2t, 2t+1) of its row, and marches
+// through a chunk of z-planes; persistent CTAs walk the (tile, z-chunk) items.
+// The 32 x 8 tile loads 2.2 halo values per cell and component (64 x 4: 2.8),
+// which is what lets three CTAs share an SM, and its 32-cell columns put fewer
+// cells into tiles that touch an x layer.
+//
+// Items come in two lists with kernels of their own.  Lean items hold no PML
+// cell and no cell outside the grid: their kernel needs 94-142 registers
+// instead of 160-240, so it keeps three (16-bit storage: four) CTAs per SM
+// where the one kernel for both kept two (three), and runs both parts of a
+// tile side by side (they share the stage input's V and sigma in L2).  The
+// march is bound by latency and instruction fetch before it is bound by HBM,
+// so resident warps count: the 400x400x200 hill's lean launch at three CTAs
+// moves 66-69% of the DRAM peak (52-58% before).  Unrolling the march by 2 or
+// 5 (no register moves in the z-window) is slower: 14.9 -> 15.2 and 16.5 ms on
+// the 600x600x250 hill; four CTAs with two slots too (15.4 ms).
 //
 // Pairs make every per-cell quantity a float2: the stencil and RHS
 // arithmetic runs as packed FFMA2 / FMUL2 / FADD2 (one instruction for both
@@ -18,14 +31,14 @@
 // (reach -1..+3) marches downwards, a backward one (reach -3..+1) upwards, so
 // the stencil always needs one plane ahead and three behind.  Each plane
 // arrives by TMA (cp.async.bulk.tensor, no multicast) into one slot of a
-// 4-slot shared-memory ring, on one mbarrier per slot:
+// shared-memory ring of 3 or 4, on one mbarrier per slot:
 //   * the differentiated components with an x/y halo, one 4-D box
-//     {72 x, 10 y, 1 z, NC components} (x from -4, y from -3);
-//   * the pointwise operands of the plane, boxes {64, 4, 1, n}: the RK
+//     {40 x, 14 y, 1 z, NC components} (x from -4, y from -3);
+//   * the pointwise operands of the plane, boxes {32, 8, 1, n}: the RK
 //     registers (FW and/or tW), the media coefficients and the metric.
 // A plane is needed one iteration after it lands (its centre enters the
 // per-thread register window of five planes) and in the next one (x/y
-// stencils, pointwise operands); two further planes are in flight.
+// stencils, pointwise operands); one or two further planes are in flight.
 //
 // The per-cell arithmetic is that of the reference's CalDiffmix + CalWavemix
 // + Iteration* (src/calculate.cu:4121-4621, 6330-6734); the top three layers'
@@ -55,7 +68,8 @@ namespace cgfd {
 namespace pair {
 using namespace ptx;
 
-constexpr int TX = 32, TY = 4, TT = TX * TY;  // threads per CTA
+constexpr int TX = 16, TY = 8, TT = TX * TY;  // threads per CTA
+constexpr int NWARP = TT / 32;
 constexpr int CX = 2 * TX;                    // cells per tile row
 constexpr int HY = TY + 6;                    // halo box rows (y from -3)
 constexpr int PWT = CX * TY;                  // values per pointwise tile
@@ -66,12 +80,10 @@ template <typename T> struct Halo {
   static constexpr int HX = CX + 2 * HOFF;
   static constexpr int HPL = HX * HY;  // values per component per halo plane
 };
-constexpr int NSLOT = 4;
 enum { PART_VEL = 0, PART_STR = 1 };
-#ifndef CGFD_PAIR_UNROLL
-#define CGFD_PAIR_UNROLL 1
-#endif
-constexpr int MARCH_UNROLL = CGFD_PAIR_UNROLL;  // unroll factor of the march loop
+// launches of a stage: the velocity and the stress part of the general items,
+// and both parts of the lean ones
+enum { GEN_VEL = PART_VEL, GEN_STR = PART_STR, LEAN_BOTH = 2, NLIST = 3 };
 
 // NC: staged (differentiated) components, C0: first of them in a set;
 // NS: components the part updates (V: 3, T: 6), S0 their first index;
@@ -100,37 +112,46 @@ template <typename T, int PART> struct Slot {
   static constexpr uint32_t COEF = U1 + up128(U_B);
   static constexpr uint32_t MET = COEF + (uint32_t)(PartInfo<PART>::NCOEF * PWT * 4);
   static constexpr uint32_t BYTES = MET + 3 * PWT * 4;
-  static constexpr size_t SMEM = (size_t)NSLOT * BYTES + 128 + 128;  // + barriers, align slack
 };
 static_assert(Slot<float, PART_VEL>::BYTES % 128 == 0 && Slot<float, PART_STR>::BYTES % 128 == 0,
               "slots");
 static_assert(Slot<__half, PART_VEL>::BYTES % 128 == 0 && Slot<__half, PART_STR>::BYTES % 128 == 0,
               "slots");
-// two CTAs per SM: 228 KB of shared memory per SM, 1 KB of it reserved per CTA
-static_assert(2 * (Slot<float, PART_VEL>::SMEM + 1024) <= 233472, "two velocity CTAs per SM");
-static_assert(2 * (Slot<float, PART_STR>::SMEM + 1024) <= 233472, "two stress CTAs per SM");
 
-// resident CTAs per SM the kernels are compiled for.  FP32 storage: two
-// (four 27.5 KB slots per CTA; registers <= 255).  16-bit storage: three
-// (the slots are about half as large; registers <= 168, a few bytes of
-// spills in some instantiations): 6.90 -> 5.79 ms per step on the
-// 400x400x200 hill with FP16 storage (with six stress auxiliaries per PML
-// direction the stress part needed 248 registers and three CTAs ran slower).
-template <typename T> struct MinCtas { static constexpr int value = 2; };
-template <> struct MinCtas<__half> { static constexpr int value = 3; };
-template <> struct MinCtas<__nv_bfloat16> { static constexpr int value = 3; };
-static_assert(3 * (Slot<__half, PART_VEL>::SMEM + 1024) <= 233472, "three 16-bit velocity CTAs");
-static_assert(3 * (Slot<__half, PART_STR>::SMEM + 1024) <= 233472, "three 16-bit stress CTAs");
+// Resident CTAs per SM the kernels are compiled for, and ring slots.  General
+// FP32: three CTAs at 168 registers with three slots, FA and tA read at the
+// update: the 256x256x128 hill 1.69 ms per step against 1.77 with two CTAs,
+// four slots and those loads early (the 160x160x80 half-space 0.53, 0.56).
+// General 16-bit: three CTAs (four would spill 120-290 B per thread: 1.88
+// instead of 1.49 ms).
+template <typename T, bool LEAN> struct Res;
+template <> struct Res<float, false> { static constexpr int CTAS = 3, NSLOT = 3; };
+template <> struct Res<float, true> { static constexpr int CTAS = 3, NSLOT = 3; };
+template <> struct Res<__half, false> { static constexpr int CTAS = 3, NSLOT = 4; };
+template <> struct Res<__half, true> { static constexpr int CTAS = 4, NSLOT = 3; };
+template <> struct Res<__nv_bfloat16, false> : Res<__half, false> {};
+template <> struct Res<__nv_bfloat16, true> : Res<__half, true> {};
+template <typename T, int LIST> struct Ring {
+  static constexpr bool LEAN = LIST == LEAN_BOTH;
+  static constexpr int NSLOT = Res<T, LEAN>::NSLOT, CTAS = Res<T, LEAN>::CTAS;
+  static constexpr uint32_t BYTES_V = Slot<T, PART_VEL>::BYTES, BYTES_S = Slot<T, PART_STR>::BYTES;
+  static constexpr uint32_t BYTES = LIST == GEN_VEL   ? BYTES_V
+                                    : LIST == GEN_STR ? BYTES_S
+                                    : BYTES_V > BYTES_S ? BYTES_V : BYTES_S;
+  static constexpr size_t SMEM = (size_t)NSLOT * BYTES + 128 + 128;  // + barriers, align slack
+  // 228 KB of shared memory per SM, 1 KB of it reserved per CTA
+  static_assert(CTAS * (SMEM + 1024) <= 233472, "resident CTAs");
+};
 
 // Tensor maps of one launch.  halo/u0/u1/coef/met feed the ring; the aux
 // maps (per direction: stage input, FA, tA) only drive L2 prefetches.
 struct Maps {
-  CUtensorMap halo;  // stage input, box {72, 10, 1, NC}
-  CUtensorMap u0;    // FW (or tW), box {64, 4, 1, NS}
-  CUtensorMap u1;    // tW, box {64, 4, 1, NS}
-  CUtensorMap coef;  // media, box {64, 4, 1, NCOEF}
-  CUtensorMap met;   // metric, box {64, 4, 1, 3}
-  CUtensorMap aux[3][3];  // [direction][ain, afw, ta], box {64, 4, 1, NS}
+  CUtensorMap halo;  // stage input, box {40, 14, 1, NC}
+  CUtensorMap u0;    // FW (or tW), box {32, 8, 1, NS}
+  CUtensorMap u1;    // tW, box {32, 8, 1, NS}
+  CUtensorMap coef;  // media, box {32, 8, 1, NCOEF}
+  CUtensorMap met;   // metric, box {32, 8, 1, 3}
+  CUtensorMap aux[3][3];  // [direction][ain, afw, ta], box {32, 8, 1, NS}
 };
 
 // Work list of a launch: items {i0, j0, z0 | z1 << 16, model} (tile
@@ -140,12 +161,14 @@ struct Maps {
 // fill the tail.  A batched launch reads each model's stage arguments and
 // tensor maps from the device arrays bargs / bmaps (one entry per model).
 struct Work {
-  const int4 *items;
-  int *counter;       // [0]: velocity launch, [1]: stress launch
-  int nitems;
+  const int4 *items[2];  // general, lean
+  // per launch: next item, CTAs done; zero between launches
+  int *counter;
+  int nitems[2];
   int has_aux[3];     // direction has a PML (aux maps valid; single model)
   const StageArgs *bargs;
-  const Maps *bmaps;
+  const Maps *bmaps;   // [velocity, stress][model]
+  int nmodels;
   // bound of every mbarrier wait, and the test hook of cgfd_test_withhold_copy:
   // with withhold >= 0 the velocity part's CTA 0 does not issue the halo copy
   // of entry `withhold` of its first item, so its wait for that plane expires
@@ -162,8 +185,24 @@ __device__ __forceinline__ f2 mul2(f2 a, f2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ f2 add2(f2 a, f2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ f2 neg2(f2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ f2 lds2(const float *p) { return *reinterpret_cast<const f2 *>(p); }
+// Reads of the ring: explicit shared-memory loads at 32-bit addresses.  The
+// slots are written by tensor copies only, which the compiler does not see as
+// stores.
+__device__ __forceinline__ f2 lds_f2(uint32_t a) {
+  f2 r;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "r"(a));
+  return r;
+}
+__device__ __forceinline__ unsigned lds_u32(uint32_t a) {
+  unsigned r;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(r) : "r"(a));
+  return r;
+}
 // a pair of stored values (any storage type) as float2
-template <typename T> __device__ __forceinline__ f2 ldp(const T *p) { return Elem<T>::ld2(p); }
+template <typename T> __device__ __forceinline__ f2 ldp(uint32_t a) {
+  if constexpr (sizeof(T) == 4) return lds_f2(a);
+  else return Elem<T>::widen(lds_u32(a));
+}
 // r times a power-of-two component scale; FP32 storage is unscaled
 template <typename T> __device__ __forceinline__ float scaled(float r, float s) {
   if constexpr (sizeof(T) == 4) return r;
@@ -172,35 +211,34 @@ template <typename T> __device__ __forceinline__ float scaled(float r, float s) 
 
 // DRP/opt MacCormack 5-point operator on a pair, in the forward form
 // (m1 = p - s, c0 = p, p1..p3 = p + s..3s for the marching sign s; r = s/h)
-__device__ __forceinline__ f2 drp2(f2 m1, f2 c0, f2 p1, f2 p2, f2 p3, float r) {
-  f2 t = mul2(S2(CGFD_DA_1), m1);
-  t = fma2(S2(CGFD_DA0), c0, t);
-  t = fma2(S2(CGFD_DA1), p1, t);
-  t = fma2(S2(CGFD_DA2), p2, t);
-  t = fma2(S2(CGFD_DA3), p3, t);
-  return mul2(t, S2(r));
+// (raw: h times the derivative; the marching sign S is in the coefficients)
+template <int S>
+__device__ __forceinline__ f2 drp2_raw(f2 m1, f2 c0, f2 p1, f2 p2, f2 p3) {
+  f2 t = mul2(S2(S * CGFD_DA_1), m1);
+  t = fma2(S2(S * CGFD_DA0), c0, t);
+  t = fma2(S2(S * CGFD_DA1), p1, t);
+  t = fma2(S2(S * CGFD_DA2), p2, t);
+  return fma2(S2(S * CGFD_DA3), p3, t);
 }
 
-// x-derivative of the pair (halo columns cb, cb+1 of row R) with the centre
-// pair C already in registers; r = X/h
+// x-derivative (raw) of the pair at ring address p (halo plane), its values C
+// already in registers
 template <int X, typename T>
-__device__ __forceinline__ f2 dx_pair(const T *R, int cb, f2 C, float r) {
+__device__ __forceinline__ f2 dx_pair(uint32_t p, f2 C) {
+  constexpr int E = sizeof(T);
   if constexpr (X > 0) {
-    const f2 La = ldp(R + cb - 2), Lb = ldp(R + cb + 2), Lc = ldp(R + cb + 4);
-    return drp2(F2(La.y, C.x), C, F2(C.y, Lb.x), Lb, F2(Lb.y, Lc.x), r);
+    const f2 La = ldp<T>(p - 2 * E), Lb = ldp<T>(p + 2 * E), Lc = ldp<T>(p + 4 * E);
+    return drp2_raw<X>(F2(La.y, C.x), C, F2(C.y, Lb.x), Lb, F2(Lb.y, Lc.x));
   } else {
-    const f2 Lz = ldp(R + cb - 4), La = ldp(R + cb - 2), Lb = ldp(R + cb + 2);
-    return drp2(F2(C.y, Lb.x), C, F2(La.y, C.x), La, F2(Lz.y, La.x), r);
+    const f2 Lz = ldp<T>(p - 4 * E), La = ldp<T>(p - 2 * E), Lb = ldp<T>(p + 2 * E);
+    return drp2_raw<X>(F2(C.y, Lb.x), C, F2(La.y, C.x), La, F2(Lz.y, La.x));
   }
 }
-// y-derivative of the pair from the component's halo plane P (row ry of
-// this thread, column cb), centre pair C in registers; r = Y/h
+// y-derivative (raw) of the same
 template <int Y, typename T>
-__device__ __forceinline__ f2 dy_pair(const T *P, int ry, int cb, f2 C, float r) {
-  constexpr int HX = Halo<T>::HX;
-  const f2 m1 = ldp(P + (ry - Y) * HX + cb), p1 = ldp(P + (ry + Y) * HX + cb);
-  const f2 p2 = ldp(P + (ry + 2 * Y) * HX + cb), p3 = ldp(P + (ry + 3 * Y) * HX + cb);
-  return drp2(m1, C, p1, p2, p3, r);
+__device__ __forceinline__ f2 dy_pair(uint32_t p, f2 C) {
+  constexpr uint32_t R = (uint32_t)(Y * Halo<T>::HX * (int)sizeof(T));  // (mod 2^32)
+  return drp2_raw<Y>(ldp<T>(p - R), C, ldp<T>(p + R), ldp<T>(p + 2u * R), ldp<T>(p + 3u * R));
 }
 
 // masked pair access: bit 0 = first cell, bit 1 = second; p1 is the second
@@ -245,41 +283,23 @@ __device__ __forceinline__ void stt2(T *p, int m, f2 v) {
 // arithmetic is that of a widened window, at half its registers (the 16-bit
 // kernels run at 168 registers to fit three CTAs per SM).
 template <typename T> struct Win {
+  using type = unsigned;
+  __device__ __forceinline__ static f2 get(unsigned v) { return Elem<T>::widen(v); }
+  __device__ __forceinline__ static unsigned ld(uint32_t a) { return lds_u32(a); }
+  // from global memory
+  __device__ __forceinline__ static unsigned ldm(const T *p, int m) {
+    if (m == 3) return *reinterpret_cast<const unsigned *>(p);
+    const unsigned short *h = reinterpret_cast<const unsigned short *>(p);
+    return ((m & 1) ? (unsigned)h[0] : 0u) | ((m & 2) ? (unsigned)h[1] << 16 : 0u);
+  }
+  __device__ __forceinline__ static unsigned zero() { return 0u; }
+};
+template <> struct Win<float> {
   using type = f2;
   __device__ __forceinline__ static f2 get(f2 v) { return v; }
-  __device__ __forceinline__ static type ld(const T *p) { return ldp(p); }
-  __device__ __forceinline__ static type ldm(const T *p, int m) { return ldt2(p, m); }
+  __device__ __forceinline__ static type ld(uint32_t a) { return lds_f2(a); }
+  __device__ __forceinline__ static type ldm(const float *p, int m) { return ldt2(p, m); }
   __device__ __forceinline__ static type zero() { return S2(0.f); }
-};
-template <> struct Win<__half> {
-  using type = __half2;
-  __device__ __forceinline__ static f2 get(__half2 v) { return __half22float2(v); }
-  __device__ __forceinline__ static type ld(const __half *p) {
-    return *reinterpret_cast<const __half2 *>(p);
-  }
-  __device__ __forceinline__ static type zero() { return __float2half2_rn(0.f); }
-  __device__ __forceinline__ static type ldm(const __half *p, int m) {
-    if (m == 3) return ld(p);
-    __half2 r = zero();
-    if (m & 1) r.x = p[0];
-    if (m & 2) r.y = p[1];
-    return r;
-  }
-};
-template <> struct Win<__nv_bfloat16> {
-  using type = __nv_bfloat162;
-  __device__ __forceinline__ static f2 get(__nv_bfloat162 v) { return __bfloat1622float2(v); }
-  __device__ __forceinline__ static type ld(const __nv_bfloat16 *p) {
-    return *reinterpret_cast<const __nv_bfloat162 *>(p);
-  }
-  __device__ __forceinline__ static type zero() { return __float2bfloat162_rn(0.f); }
-  __device__ __forceinline__ static type ldm(const __nv_bfloat16 *p, int m) {
-    if (m == 3) return ld(p);
-    __nv_bfloat162 r = zero();
-    if (m & 1) r.x = p[0];
-    if (m & 2) r.y = p[1];
-    return r;
-  }
 };
 
 // 16-bit storage keeps the RK accumulator as its difference from the step
@@ -321,20 +341,13 @@ __device__ __forceinline__ void rk_store2(const StageArgs &a, T *out, T *tw, int
 
 // ADE auxiliaries of one pair and direction: the stage input ai (FA in the
 // first stage, A after) enters the RHS and is loaded before the stencil
-// arithmetic.  EARLY (FP32 storage, which has the registers): the RK
-// registers of the update (FA and tA in the inner stages, tA in the final
-// one) are loaded with it, so the boundary path pays one memory round trip
-// per plane, hidden behind the stencil.  Otherwise (16-bit storage, three
-// CTAs per SM at 168 registers) the update reads FA and tA of one direction
-// right before writing A (FA in the final stage) and tA, so only one
-// direction's values are live; loading them early there doubled the spills.
+// arithmetic.  The update reads FA and tA of one direction right before
+// writing A (FA in the final stage) and tA, so that only one direction's
+// values are live at the 168 registers that three CTAs per SM leave.
 // o0/o1: the cells' indices, m: the cells' mask.
-template <int KIND, int N, bool EARLY>
+template <int KIND, int N>
 struct Aux2 {
-  static constexpr int NU = (KIND == 0 || !EARLY) ? 1 : N, NV = (KIND == 1 && EARLY) ? N : 1;
   f2 ai[N];
-  f2 u[NU];  // EARLY: FA (inner stages) or tA (final stage)
-  f2 v[NV];  // EARLY: tA (inner stages)
   __device__ __forceinline__ void load(const StageArgs &a, int d, size_t o0, size_t o1, int m,
                                        int c0) {
     const size_t as = a.g.astride[d];
@@ -342,14 +355,6 @@ struct Aux2 {
     for (int q = 0; q < N; ++q) {
       const float *b = a.ain[d] + (c0 + q) * as;
       ai[q] = ld2(b + o0, b + o1, m);
-      if constexpr (EARLY && KIND == 1) {
-        const float *f = a.afw[d] + (c0 + q) * as, *t = a.ta[d] + (c0 + q) * as;
-        u[q] = ld2(f + o0, f + o1, m);
-        v[q] = ld2(t + o0, t + o1, m);
-      } else if constexpr (EARLY && KIND == 2) {
-        const float *t = a.ta[d] + (c0 + q) * as;
-        u[q] = ld2(t + o0, t + o1, m);
-      }
     }
   }
   __device__ __forceinline__ void update(const StageArgs &a, int d, size_t o0, size_t o1, int m,
@@ -361,17 +366,6 @@ struct Aux2 {
         float *po = a.aout[d] + (c0 + q) * as, *pt = a.ta[d] + (c0 + q) * as;
         st2(po + o0, po + o1, m, fma2(S2(a.adt), hh[q], ai[q]));
         st2(pt + o0, pt + o1, m, fma2(S2(a.bdt), hh[q], ai[q]));
-      }
-    } else if constexpr (EARLY) {
-#pragma unroll
-      for (int q = 0; q < N; ++q) {
-        float *po = a.aout[d] + (c0 + q) * as, *pt = a.ta[d] + (c0 + q) * as;
-        if (KIND == 1) {
-          st2(po + o0, po + o1, m, fma2(S2(a.adt), hh[q], u[q]));
-          st2(pt + o0, pt + o1, m, fma2(S2(a.bdt), hh[q], v[q]));
-        } else {
-          st2(po + o0, po + o1, m, fma2(S2(a.bdt), hh[q], u[q]));
-        }
       }
     } else if constexpr (KIND == 1) {
       // FA and tA together: one memory round trip per direction
@@ -421,7 +415,7 @@ struct Pair {
 struct Plane {
   int iz, k;
   size_t c;           // linear index of the first cell
-  bool zpml, top, near_top, curved, lean;
+  bool zpml, top, near_top, curved;
   bool met;           // the plane's metric tile was loaded
   float zz;           // zeta_z of the plane when no tile was loaded
   // zeta_z of this thread's pair
@@ -430,15 +424,15 @@ struct Plane {
   }
 };
 
-// Pointwise operands of this thread's pair in the current slot.
+// Pointwise operands of this thread's pair in the current slot (ring
+// addresses).
 template <typename T>
 struct Pw2 {
-  const T *u0, *u1;
-  const float *coef, *met;
-  __device__ f2 U0(int q) const { return ldp(u0 + q * PWT); }
-  __device__ f2 U1(int q) const { return ldp(u1 + q * PWT); }
-  __device__ f2 C(int q) const { return lds2(coef + q * PWT); }
-  __device__ f2 M(int q) const { return lds2(met + q * PWT); }
+  uint32_t u0, u1, coef, met;
+  __device__ f2 U0(int q) const { return ldp<T>(u0 + q * PWT * (int)sizeof(T)); }
+  __device__ f2 U1(int q) const { return ldp<T>(u1 + q * PWT * (int)sizeof(T)); }
+  __device__ f2 C(int q) const { return lds_f2(coef + q * PWT * 4); }
+  __device__ f2 M(int q) const { return lds_f2(met + q * PWT * 4); }
 };
 
 // auxiliary indices of the pair on a plane (X: per cell; Y, Z: the pair is
@@ -467,55 +461,83 @@ struct AuxIdx {
 // layers' velocities come from the traction-image kernel (timg.cu); only
 // their z auxiliaries are updated here.
 // w[s][q]: staged component s on plane iz + (3 - q) * Z (q = 3: this plane).
-template <typename T, int X, int Y, int Z, int KIND>
+template <typename T, int X, int Y, int Z, int KIND, bool LEAN>
 __device__ __forceinline__ void vel_pair(const StageArgs &a, const Pair &e, const Plane &pl,
-                                         const T *H, int ry, int cb, const Pw2<T> &pw,
-                                         const typename Win<T>::type (&w)[6][5], float rx,
-                                         float rys, float rz) {
-  constexpr int HX = Halo<T>::HX, HPL = Halo<T>::HPL;
+                                         uint32_t hp, const Pw2<T> &pw,
+                                         const typename Win<T>::type (&w)[6][5],
+                                         float rh) {
+  constexpr uint32_t HPB = Halo<T>::HPL * sizeof(T);
   const size_t fs = a.g.fstride;
   auto W = [&](int s, int q) { return Win<T>::get(w[s][q]); };
   // 1/h factors carry the staged component's scale (stored units -> values)
-  auto sr = [&](float r, int s) { return scaled<T>(r, a.sc[TXX + s]); };
-  auto dx = [&](int s) { return dx_pair<X>(H + s * HPL + ry * HX, cb, W(s, 3), sr(rx, s)); };
-  auto dy = [&](int s) { return dy_pair<Y>(H + s * HPL, ry, cb, W(s, 3), sr(rys, s)); };
-  auto dz = [&](int s) {
-    return drp2(W(s, 4), W(s, 3), W(s, 2), W(s, 1), W(s, 0), sr(rz, s));
-  };
+  auto sr = [&](int s) { return S2(scaled<T>(rh, a.sc[TXX + s])); };
+  auto dx_raw = [&](int s) { return dx_pair<X, T>(hp + s * HPB, W(s, 3)); };
+  auto dy_raw = [&](int s) { return dy_pair<Y, T>(hp + s * HPB, W(s, 3)); };
+  auto dz_raw = [&](int s) { return drp2_raw<Z>(W(s, 4), W(s, 3), W(s, 2), W(s, 1), W(s, 0)); };
+  auto dx = [&](int s) { return mul2(dx_raw(s), sr(s)); };
+  auto dy = [&](int s) { return mul2(dy_raw(s), sr(s)); };
+  auto dz = [&](int s) { return mul2(dz_raw(s), sr(s)); };
   T *out = static_cast<T *>(a.out), *tw = static_cast<T *>(a.tw);
   auto adt = [&](int c) { return scaled<T>(a.adt, a.isc[c]); };
   auto bdt = [&](int c) { return scaled<T>(a.bdt, a.isc[c]); };
 
-  if (pl.lean) {
+  if constexpr (LEAN) {
+    // components of the stress set: Txx Tyy Tzz Txy Txz Tyz
+    constexpr int SX[3] = {0, 3, 4}, SY[3] = {3, 1, 5}, SZ[3] = {4, 5, 2};
     const f2 irho = pw.C(0);
     const f2 ztz = pl.zeta_z(pw);
     f2 hw[3];
-    if (pl.curved) {
-      const f2 ztx = pw.M(0), zty = pw.M(1);
-      const f2 DzTxx = dz(0), DzTyy = dz(1), DzTzz = dz(2);
-      const f2 DzTxy = dz(3), DzTxz = dz(4), DzTyz = dz(5);
-      const f2 z0 = mul2(fma2(ztz, DzTxz, fma2(zty, DzTxy, mul2(ztx, DzTxx))), irho);
-      const f2 z1 = mul2(fma2(ztz, DzTyz, fma2(zty, DzTyy, mul2(ztx, DzTxy))), irho);
-      const f2 z2 = mul2(fma2(ztz, DzTzz, fma2(zty, DzTyz, mul2(ztx, DzTxz))), irho);
-      hw[0] = add2(add2(mul2(dx(0), irho), mul2(dy(3), irho)), z0);
-      hw[1] = add2(add2(mul2(dx(3), irho), mul2(dy(1), irho)), z1);
-      hw[2] = add2(add2(mul2(dx(4), irho), mul2(dy(5), irho)), z2);
+    if constexpr (sizeof(T) == 4) {
+      // raw derivatives, 1/(rho h) once per component
+      const f2 ir = mul2(irho, S2(rh));
+      if (pl.curved) {
+        const f2 ztx = pw.M(0), zty = pw.M(1);
+        f2 z[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) z[q] = dz_raw(q);
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          hw[q] = mul2(fma2(ztz, z[SZ[q]],
+                            fma2(zty, z[SY[q]], fma2(ztx, z[SX[q]], add2(dx_raw(SX[q]), dy_raw(SY[q]))))),
+                       ir);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          hw[q] = mul2(fma2(ztz, dz_raw(SZ[q]), add2(dx_raw(SX[q]), dy_raw(SY[q]))), ir);
+      }
     } else {
-      hw[0] = add2(add2(mul2(dx(0), irho), mul2(dy(3), irho)), mul2(mul2(ztz, dz(4)), irho));
-      hw[1] = add2(add2(mul2(dx(3), irho), mul2(dy(1), irho)), mul2(mul2(ztz, dz(5)), irho));
-      hw[2] = add2(add2(mul2(dx(4), irho), mul2(dy(5), irho)), mul2(mul2(ztz, dz(2)), irho));
+      // scaled derivatives (16-bit storage has a scale per component), and sums
+      // of the rounded products as in the general path with B = 1 (a plain add2 of
+      // products would be contracted)
+      const f2 one = S2(a.one);
+      f2 zs[3];
+      if (pl.curved) {
+        const f2 ztx = pw.M(0), zty = pw.M(1);
+        f2 z[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) z[q] = dz(q);
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          zs[q] = fma2(ztz, z[SZ[q]], fma2(zty, z[SY[q]], mul2(ztx, z[SX[q]])));
+      } else {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) zs[q] = mul2(ztz, dz(SZ[q]));
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        hw[q] = fma2(mul2(zs[q], irho), one,
+                     fma2(mul2(dx(SX[q]), irho), one, mul2(dy(SY[q]), irho)));
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q)
       rk_store2<KIND>(a, out + (VX + q) * fs + pl.c, tw + (VX + q) * fs + pl.c, 3, pw.U0(q),
                       TwoRegs<KIND, T>::value ? pw.U1(q) : S2(0.f), hw[q], adt(VX + q), bdt(VX + q));
     return;
-  }
-
+  } else {
   // general path: issue every auxiliary load before the stencil arithmetic
   const AuxIdx ix(a, e, pl);
   const int mx = e.mx, my = e.ypml ? e.m : 0, mz = pl.zpml ? e.m : 0;
-  Aux2<KIND, 3, sizeof(T) == 4> ax, ay, az;
+  Aux2<KIND, 3> ax, ay, az;
   if (mx) ax.load(a, 0, ix.x0, ix.x1, mx, 0);
   if (my) ay.load(a, 1, ix.y, ix.y + 1, my, 0);
   if (mz) az.load(a, 2, ix.z, ix.z + 1, mz, 0);
@@ -573,11 +595,12 @@ __device__ __forceinline__ void vel_pair(const StageArgs &a, const Pair &e, cons
   if (mxs) ax.update(a, 0, ix.x0, ix.x1, mxs, 0, hax);
   if (mys) ay.update(a, 1, ix.y, ix.y + 1, mys, 0, hay);
   if (mz) az.update(a, 2, ix.z, ix.z + 1, mz, 0, haz);
-  if (!xy) return;
+  const int ms = xy ? e.m : 0;
 #pragma unroll
   for (int q = 0; q < 3; ++q)
-    rk_store2<KIND>(a, out + (VX + q) * fs + pl.c, tw + (VX + q) * fs + pl.c, e.m, pw.U0(q),
+    rk_store2<KIND>(a, out + (VX + q) * fs + pl.c, tw + (VX + q) * fs + pl.c, ms, pw.U0(q),
                     TwoRegs<KIND, T>::value ? pw.U1(q) : S2(0.f), hw[q], adt(VX + q), bdt(VX + q));
+  }
 }
 
 // --------------------------- stress part ----------------------------------
@@ -592,43 +615,90 @@ __device__ __forceinline__ f2 mat_row(const float *mv, size_t plane, int r, f2 u
               fma2(lds2(mv + (r + 1) * plane), v, mul2(lds2(mv + r * plane), u)));
 }
 
-template <typename T, int X, int Y, int Z, int KIND>
+template <typename T, int X, int Y, int Z, int KIND, bool LEAN>
 __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, const Plane &pl,
-                                         const T *H, int ry, int cb, const Pw2<T> &pw,
-                                         const typename Win<T>::type (&w)[3][5], float rx,
-                                         float rys, float rz) {
-  constexpr int HX = Halo<T>::HX, HPL = Halo<T>::HPL;
+                                         uint32_t hp, const Pw2<T> &pw,
+                                         const typename Win<T>::type (&w)[3][5],
+                                         float rh) {
+  constexpr uint32_t HPB = Halo<T>::HPL * sizeof(T);
   const Geom &g = a.g;
   auto W = [&](int s, int q) { return Win<T>::get(w[s][q]); };
   const size_t fs = g.fstride;
   // 1/h factors carry the staged component's scale (stored units -> values)
-  auto sr = [&](float r, int s) { return scaled<T>(r, a.sc[VX + s]); };
-  auto dx = [&](int s) { return dx_pair<X>(H + s * HPL + ry * HX, cb, W(s, 3), sr(rx, s)); };
-  auto dy = [&](int s) { return dy_pair<Y>(H + s * HPL, ry, cb, W(s, 3), sr(rys, s)); };
-  auto dz = [&](int s) {
-    return drp2(W(s, 4), W(s, 3), W(s, 2), W(s, 1), W(s, 0), sr(rz, s));
-  };
+  auto sr = [&](int s) { return S2(scaled<T>(rh, a.sc[VX + s])); };
+  auto dx_raw = [&](int s) { return dx_pair<X, T>(hp + s * HPB, W(s, 3)); };
+  auto dy_raw = [&](int s) { return dy_pair<Y, T>(hp + s * HPB, W(s, 3)); };
+  auto dz_raw = [&](int s) { return drp2_raw<Z>(W(s, 4), W(s, 3), W(s, 2), W(s, 1), W(s, 0)); };
+  auto dx = [&](int s) { return mul2(dx_raw(s), sr(s)); };
+  auto dy = [&](int s) { return mul2(dy_raw(s), sr(s)); };
+  auto dz = [&](int s) { return mul2(dz_raw(s), sr(s)); };
   T *out = static_cast<T *>(a.out), *tw = static_cast<T *>(a.tw);
 
+  if constexpr (LEAN) {
+    // FP32: raw derivatives, the moduli carry 1/h.  16-bit storage has a scale
+    // per component, which the derivatives carry with 1/h.
+    constexpr bool RAW = sizeof(T) == 4;
+    auto gx = [&](int s) { return RAW ? dx_raw(s) : dx(s); };
+    auto gy = [&](int s) { return RAW ? dy_raw(s) : dy(s); };
+    auto sz = [&](int s) { return RAW ? S2((float)Z) : mul2(S2((float)Z), sr(s)); };
+    const f2 DxVx = gx(0), DxVy = gx(1), DxVz = gx(2);
+    const f2 DyVx = gy(0), DyVy = gy(1), DyVz = gy(2);
+    f2 DzV[3];
+    if (pl.iz < g.top - 2) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) DzV[q] = RAW ? dz_raw(q) : dz(q);
+    } else if (pl.top) {
+      const float *mv = a.matv + (size_t)e.iy * g.px + e.ix;
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        DzV[q] = add2(mat_row(mv + 9 * g.plane, g.plane, 3 * q, DyVx, DyVy, DyVz),
+                      mat_row(mv, g.plane, 3 * q, DxVx, DxVy, DxVz));
+    } else if (pl.iz == g.top - 1) {  // 2-point (M22)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) DzV[q] = mul2(add2(W(q, 2), neg2(W(q, 3))), sz(q));
+    } else {  // Gottlieb 2-4 (M24)
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        DzV[q] = mul2(fma2(S2(CGFD_MA2), W(q, 1),
+                           fma2(S2(CGFD_MA1), W(q, 2), mul2(S2(CGFD_MA0), W(q, 3)))), sz(q));
+    }
+    const f2 rr = S2(RAW ? rh : 1.f);
+    const f2 mu = mul2(pw.C(1), rr), mu2 = add2(mu, mu);
+    const f2 lam = fma2(pw.C(0), rr, neg2(mu2));
+    const f2 ztz = pl.zeta_z(pw);
+    // sigma_kk: lambda * (trace of the gradient) + 2 mu * its diagonal
+    f2 ga = DxVx, gb = DyVy, gxy = add2(DxVy, DyVx), gxz = DxVz, gyz = DyVz;
+    const f2 gc = mul2(ztz, DzV[2]);
+    if (pl.curved) {
+      const f2 ztx = pw.M(0), zty = pw.M(1);
+      ga = fma2(ztx, DzV[0], ga);
+      gb = fma2(zty, DzV[1], gb);
+      gxy = fma2(ztx, DzV[1], fma2(zty, DzV[0], gxy));
+      gxz = fma2(ztx, DzV[2], gxz);
+      gyz = fma2(zty, DzV[2], gyz);
+    }
+    const f2 tr = mul2(lam, add2(add2(ga, gb), gc));
+    const f2 hw[6] = {fma2(mu2, ga, tr), fma2(mu2, gb, tr), fma2(mu2, gc, tr), mul2(mu, gxy),
+                      mul2(mu, fma2(ztz, DzV[0], gxz)), mul2(mu, fma2(ztz, DzV[1], gyz))};
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+      rk_store2<KIND>(a, out + (TXX + q) * fs + pl.c, tw + (TXX + q) * fs + pl.c, 3, pw.U0(q),
+                      TwoRegs<KIND, T>::value ? pw.U1(q) : S2(0.f), hw[q],
+                      scaled<T>(a.adt, a.isc[TXX + q]), scaled<T>(a.bdt, a.isc[TXX + q]));
+    return;
+  } else {
   // general path: issue every stage-input auxiliary load before the stencil.
   // The stress auxiliaries are kept as one per velocity derivative of the
   // direction (x: d/dx of Vx, Vy, Vz; y: d/dy; z: d/dzeta): each stress's
   // ADE auxiliary is the same linear combination of them, with cell-constant
   // coefficients, as its RHS term is of the derivatives (the ADE is linear),
   // so three values per direction stand for six.
-  const bool gen = !pl.lean;
-  int mx = 0, my = 0, mz = 0;
-  AuxIdx ix;
-  Aux2<KIND, 3, sizeof(T) == 4> ax, ay, az;
-  if (gen) {
-    ix = AuxIdx(a, e, pl);
-    mx = e.mx;
-    my = e.ypml ? e.m : 0;
-    mz = pl.zpml ? e.m : 0;
-    if (mx) ax.load(a, 0, ix.x0, ix.x1, mx, 3);
-    if (my) ay.load(a, 1, ix.y, ix.y + 1, my, 3);
-    if (mz) az.load(a, 2, ix.z, ix.z + 1, mz, 3);
-  }
+  Aux2<KIND, 3> ax, ay, az;
+  const AuxIdx ix(a, e, pl);
+  const int mx = e.mx, my = e.ypml ? e.m : 0, mz = pl.zpml ? e.m : 0;
+  if (mx) ax.load(a, 0, ix.x0, ix.x1, mx, 3);
+  if (my) ay.load(a, 1, ix.y, ix.y + 1, my, 3);
+  if (mz) az.load(a, 2, ix.z, ix.z + 1, mz, 3);
   const f2 DxVx = dx(0), DxVy = dx(1), DxVz = dx(2);
   const f2 DyVx = dy(0), DyVy = dy(1), DyVz = dy(2);
   f2 DzVx, DzVy, DzVz;
@@ -642,13 +712,17 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
     DzVz = add2(mat_row(mv + 9 * g.plane, g.plane, 6, DyVx, DyVy, DyVz),
                 mat_row(mv, g.plane, 6, DxVx, DxVy, DxVz));
   } else if (pl.iz == g.top - 1) {  // 2-point (M22)
-    DzVx = mul2(add2(W(0, 2), neg2(W(0, 3))), S2(sr(rz, 0)));
-    DzVy = mul2(add2(W(1, 2), neg2(W(1, 3))), S2(sr(rz, 1)));
-    DzVz = mul2(add2(W(2, 2), neg2(W(2, 3))), S2(sr(rz, 2)));
+    auto m22 = [&](int s) {
+      return mul2(add2(W(s, 2), neg2(W(s, 3))), mul2(S2((float)Z), sr(s)));
+    };
+    DzVx = m22(0);
+    DzVy = m22(1);
+    DzVz = m22(2);
   } else if (pl.iz == g.top - 2) {  // Gottlieb 2-4 (M24)
     auto m24 = [&](int s) {
       return mul2(fma2(S2(CGFD_MA2), W(s, 1), fma2(S2(CGFD_MA1), W(s, 2),
-                                                  mul2(S2(CGFD_MA0), W(s, 3)))), S2(sr(rz, s)));
+                                                  mul2(S2(CGFD_MA0), W(s, 3)))),
+                  mul2(S2((float)Z), sr(s)));
     };
     DzVx = m24(0);
     DzVy = m24(1);
@@ -683,10 +757,7 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
   }
 
   f2 hw[6];
-  if (!gen) {
-#pragma unroll
-    for (int q = 0; q < 6; ++q) hw[q] = add2(add2(dxi[q], det[q]), dzt[q]);
-  } else {
+  {
     const f2 iBy = S2(e.iBy), iBz = S2(ix.iBz);
 #pragma unroll
     for (int q = 0; q < 6; ++q)
@@ -768,158 +839,138 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
       az.update(a, 2, ix.z, ix.z + 1, mz, 3, ha);
     }
   }
-  const int m = gen ? e.m : 3;
+  const int m = e.m;
 #pragma unroll
   for (int q = 0; q < 6; ++q)
     rk_store2<KIND>(a, out + (TXX + q) * fs + pl.c, tw + (TXX + q) * fs + pl.c, m, pw.U0(q),
                     TwoRegs<KIND, T>::value ? pw.U1(q) : S2(0.f), hw[q], scaled<T>(a.adt, a.isc[TXX + q]),
                     scaled<T>(a.bdt, a.isc[TXX + q]));
+  }
 }
 
 // ------------------------------ the march ---------------------------------
-// items: tile index fastest, so the CTAs resident at one time work on
-// neighbouring tiles of the same z-chunk and share halo rows in L2
-template <typename T, int PART, int X, int Y, int Z, int KIND, bool B>
-__global__ void __launch_bounds__(TT, MinCtas<T>::value)
-    pair_kernel(const __grid_constant__ Maps maps, const StageArgs a, const Work wk, int *err) {
+// State of a CTA's ring: the mbarrier phases and the copies in flight.
+struct RingState {
+  uint32_t ph = 0;    // parity of the next wait, per slot (same in every thread)
+  uint32_t pend = 0;  // slots with copies not yet waited for (same in every thread)
+};
+
+// One work item of one part.  Returns with every read of the ring done and
+// every copy landed, or with *abort_flag set (read after a barrier, so every
+// thread sees it).
+//
+// LEAN items lie inside the layers' inner faces: no auxiliaries, B = 1, every
+// cell of the tile valid.
+template <typename T, int PART, int X, int Y, int Z, int KIND, bool LEAN>
+__device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const Work &wk,
+                                      const bool (&aux_on)[3], const int4 it, bool withhold_item,
+                                      unsigned char *ring, uint64_t *bars, RingState &rs,
+                                      volatile int *abort_flag) {
   using S = Slot<T, PART>;
+  constexpr int NSLOT = Res<T, LEAN>::NSLOT;
   constexpr int HOFF = Halo<T>::HOFF, HX = Halo<T>::HX, HPL = Halo<T>::HPL;
   constexpr int NC = PartInfo<PART>::NC, C0 = PartInfo<PART>::C0;
   constexpr int S0 = PartInfo<PART>::S0;
   constexpr int NCOEF = PartInfo<PART>::NCOEF, COEF0 = PartInfo<PART>::COEF0;
   constexpr int DIR = (Z > 0) ? -1 : 1;  // march direction in z
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  // align the ring on the shared-window address itself
-  unsigned char *sbase = smem_raw + ((128u - (su32(smem_raw) & 127u)) & 127u);
-  unsigned char *ring = sbase;  // NSLOT slots of S::BYTES
-  uint64_t *bars = reinterpret_cast<uint64_t *>(sbase + (size_t)NSLOT * S::BYTES);
-  __shared__ int abort_flag;
-
+  constexpr int kinda = (KIND == 1) ? 3 : (KIND == 2 ? 2 : 1);  // aux sets read
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
+  const int warp = tid >> 5;
+  const bool leader = (tid & 31) == 0;
+  // this pair inside a halo plane and a pointwise tile (byte offsets)
+  const uint32_t sc = (uint32_t)(((ty + 3) * HX + HOFF + 2 * tx) * (int)sizeof(T));
+  const uint32_t tc = (uint32_t)(ty * CX + 2 * tx);
+  const uint32_t ring32 = su32(ring);
+  const Geom &g = A.g;
+  const size_t fs = g.fstride;
+  const bool flat = A.flat;
+  auto met_tile = [&](int p) { return !flat && p >= A.zu_end; };
+  // zeta_z of a plane without a metric tile (loaded one plane ahead)
+  auto zz_of = [&](int p) { return flat ? 1.f : (p < A.zu_end ? A.zzp[p] : 0.f); };
+  const float rh = 1.f / A.h;
+  const int zlo = LFD + g.nabs[4], zhi = g.nk + LFD - g.nabs[5];  // z interior [zlo, zhi)
+  const int i0 = it.x, j0 = it.y, z0 = it.z;
+  // the traction image owns the top three layers' velocities
+  const int z1 = (LEAN && PART == PART_VEL) ? min(it.w, g.top - 2) : it.w;
+  const int n = z1 - z0;                   // planes computed
+  if (n <= 0) return;
+  const int zf = (DIR > 0) ? z0 : z1 - 1;  // first plane in march order
 
-  if (tid == 0) {
-    abort_flag = 0;
-    bool aligned = ((su32(bars) & 7u) == 0);
-    for (int s = 0; s < NSLOT; ++s)
-      aligned = aligned && ((su32(ring + (size_t)s * S::BYTES) & 127u) == 0);
-    if (!aligned) {
-      abort_flag = 1;
-      if (err) atomicExch(err, 2);
-    } else {
-      for (int s = 0; s < NSLOT; ++s) mbar_init(&bars[s], 1);
-      fence_mbar_init();
-    }
-  }
-  __syncthreads();
-  if (abort_flag) return;  // nothing was issued
-
-  uint32_t ph = 0;    // parity of the next wait, per slot (same in every thread)
-  uint32_t pend = 0;  // thread 0: slots with a copy not yet waited for
-  const int ry = ty + 3, cb = HOFF + 2 * tx;
-  const int sc = ry * HX + cb;       // this pair inside a halo plane
-  const int tc = ty * CX + 2 * tx;   // this pair inside a pointwise tile
-  const int kinda = (KIND == 1) ? 3 : (KIND == 2 ? 2 : 1);        // aux sets read
-
-  __shared__ int s_next;
-  int base = 0;  // stream position of the current item's entry 0
-  for (;;) {
-    // the next item, taken only when this CTA is free (a CTA never holds a
-    // claim on work while it is still busy)
-    if (tid == 0) s_next = atomicAdd(wk.counter + PART, 1);
-    __syncthreads();
-    const int cur = s_next;
-    if (cur >= wk.nitems || abort_flag) break;  // CTA-uniform
-    const int4 it4 = wk.items[cur];
-    const int model = B ? it4.w : 0;
-    // a batched launch reads the item's model's stage arguments in place
-    // (global memory, read-only during the launch).  Copied per item into a
-    // __shared__ StageArgs and read from there, the 16-bit batched stages
-    // behaved as if every component scale were zero (FP32, whose kernels
-    // never read the scales, was unaffected); read through a pointer to the
-    // copy hidden from the compiler they were correct but 15% slower than
-    // in place.
-    const StageArgs &A = B ? wk.bargs[model] : a;
-    const Maps &M = B ? wk.bmaps[model] : maps;
-    const Geom &g = A.g;
-    const size_t fs = g.fstride;
-    const bool flat = A.flat;
-    // bytes one plane delivers: halo always, pointwise only for computed
-    // planes, the metric tile only where the plane's metric is not uniform
-    const uint32_t pw_bytes =
-        S::U_B * (TwoRegs<KIND, T>::value ? 2u : 1u) + (uint32_t)(PWT * 4) * NCOEF;
-    auto met_tile = [&](int p) { return !flat && p >= A.zu_end; };
-    // zeta_z of a plane without a metric tile (loaded one plane ahead)
-    auto zz_of = [&](int p) { return flat ? 1.f : (p < A.zu_end ? A.zzp[p] : 0.f); };
-    const float rx = (float)X / A.h, rys = (float)Y / A.h, rz = (float)Z / A.h;
-    const int zlo = LFD + g.nabs[4], zhi = g.nk + LFD - g.nabs[5];  // z interior [zlo, zhi)
-    const bool aux_on[3] = {B ? A.ain[0] != nullptr : wk.has_aux[0] != 0,
-                         B ? A.ain[1] != nullptr : wk.has_aux[1] != 0,
-                         B ? A.ain[2] != nullptr : wk.has_aux[2] != 0};
-    const int4 it = make_int4(it4.x, it4.y, it4.z & 0xffff, it4.z >> 16);
-    const int i0 = it.x, j0 = it.y, z0 = it.z, z1 = it.w;
-    const int n = z1 - z0;                  // planes computed (>= 4)
-    const int zf = (DIR > 0) ? z0 : z1 - 1;  // first plane in march order
-    // Item entries q = 0..n (plane zf + DIR*q; entry n is read for the window
-    // only) go to ring slot (base + q) & 3, base counting the entries of the
-    // CTA's earlier items; thread 0 issues, every thread waits, in order.
-    auto issue = [&](const int4 it, int q, int s) {  // thread 0 only
-      unsigned char *slot = ring + (size_t)s * S::BYTES;
-      const int i0 = it.x, j0 = it.y, n = it.w - it.z;
-      const int p = ((DIR > 0) ? it.z : it.w - 1) + DIR * q;
-      const bool compute = q < n;
-      fence_proxy_async();
-      const bool met = compute && met_tile(p);
-      mbar_expect_tx(&bars[s], S::HALO_B + (compute ? pw_bytes : 0u) +
-                                   (met ? (uint32_t)(PWT * 4) * 3u : 0u));
-      const bool withheld = PART == PART_VEL && wk.withhold == q && base == 0 &&
-                            blockIdx.x == 0;
+  // Entry q = 0..n (plane zf + DIR*q; entry n is read for the window only)
+  // goes to ring slot q % NSLOT.  The copies of an entry are shared out over
+  // the warps' leaders, each of which adds its bytes to the slot's barrier:
+  // issued by one thread they held that thread's warp, and at the next
+  // barrier the CTA, for the length of five tensor copies and the prefetches.
+  auto issue = [&](int q, int s) {
+    rs.pend |= 1u << s;
+    if (!leader) return;
+    unsigned char *slot = ring + (size_t)s * S::BYTES;
+    const int p = zf + DIR * q;
+    const bool compute = q < n;
+    const int cx = XO + i0, cy = LFD + j0;
+    fence_proxy_async();
+    if (warp == 0) {
+      mbar_expect_tx(&bars[s], S::HALO_B);
+      const bool withheld = PART == PART_VEL && withhold_item && wk.withhold == q;
       if (!withheld) tma_load(slot, &M.halo, XO + i0 - HOFF, j0, p, C0, &bars[s]);
-      if (compute) {
-        const int cx = XO + i0, cy = LFD + j0;
-        tma_load(slot + S::U0, &M.u0, cx, cy, p, S0, &bars[s]);
-        if (TwoRegs<KIND, T>::value) tma_load(slot + S::U1, &M.u1, cx, cy, p, S0, &bars[s]);
-        tma_load(slot + S::COEF, &M.coef, cx, cy, p, COEF0, &bars[s]);
-        if (met) tma_load(slot + S::MET, &M.met, cx, cy, p, 0, &bars[s]);
-        // the plane's PML auxiliaries into L2 (tile- and plane-uniform presence)
-        const bool xp = aux_on[0] && (i0 < g.nabs[0] || i0 + CX > g.ni - g.nabs[1]);
-        const bool yp = aux_on[1] && (j0 < g.nabs[2] || j0 + TY > g.nj - g.nabs[3]);
-        const bool zp = aux_on[2] && (p < zlo || p >= zhi);
-        if (xp || yp || zp) {
-          const int xa_t = (i0 < g.nabs[0]) ? max(i0, 0) : i0 - (g.ni - g.nabs[1]) + g.xaoff;
-          const int ya_t = (j0 < g.nabs[2]) ? j0 : j0 - (g.nj - g.nabs[3]) + g.nabs[2];
-          const int za = (p - LFD < g.nabs[4]) ? p - LFD : p - LFD - (g.nk - g.nabs[5]) + g.nabs[4];
-          const int c0 = (PART == PART_VEL) ? 0 : 3;
-          const int cxp = max(cx, 0);  // prefetch boxes start inside the arrays
-          for (int t = 0; t < kinda; ++t) {
-            const int set = (KIND == 2 && t == 1) ? 2 : t;  // final stage: ain, ta
-            if (xp) tma_prefetch(&M.aux[0][set], xa_t, cy, p, c0);
-            if (yp) tma_prefetch(&M.aux[1][set], cxp, ya_t, p, c0);
-            if (zp) tma_prefetch(&M.aux[2][set], cxp, cy, za, c0);
-          }
-        }
+    } else if (warp == 1) {
+      mbar_expect_tx(&bars[s], compute ? S::U_B : 0u);
+      if (compute) tma_load(slot + S::U0, &M.u0, cx, cy, p, S0, &bars[s]);
+    } else if (warp == 2) {
+      const bool u1 = compute && TwoRegs<KIND, T>::value;
+      mbar_expect_tx(&bars[s], u1 ? S::U_B : 0u);
+      if (u1) tma_load(slot + S::U1, &M.u1, cx, cy, p, S0, &bars[s]);
+    } else {
+      const bool met = compute && met_tile(p);
+      mbar_expect_tx(&bars[s], (compute ? (uint32_t)(PWT * 4) * NCOEF : 0u) +
+                                   (met ? (uint32_t)(PWT * 4) * 3u : 0u));
+      if (compute) tma_load(slot + S::COEF, &M.coef, cx, cy, p, COEF0, &bars[s]);
+      if (met) tma_load(slot + S::MET, &M.met, cx, cy, p, 0, &bars[s]);
+    }
+    if constexpr (!LEAN) {
+      // the plane's PML auxiliaries into L2 (tile- and plane-uniform presence)
+      if (!compute || warp == 0) return;
+      const int d = warp - 1;  // direction
+      const int c0 = (PART == PART_VEL) ? 0 : 3;
+      const int cxp = max(cx, 0);  // prefetch boxes start inside the arrays
+      const bool on = aux_on[d] &&
+                      (d == 0   ? (i0 < g.nabs[0] || i0 + CX > g.ni - g.nabs[1])
+                       : d == 1 ? (j0 < g.nabs[2] || j0 + TY > g.nj - g.nabs[3])
+                                : (p < zlo || p >= zhi));
+      if (!on) return;
+      const int bx = d == 0 ? ((i0 < g.nabs[0]) ? max(i0, 0) : i0 - (g.ni - g.nabs[1]) + g.xaoff)
+                            : cxp;
+      const int by = d == 1 ? ((j0 < g.nabs[2]) ? max(j0, 0) : j0 - (g.nj - g.nabs[3]) + g.nabs[2]) : cy;
+      const int bz = d == 2 ? ((p - LFD < g.nabs[4]) ? p - LFD
+                                                     : p - LFD - (g.nk - g.nabs[5]) + g.nabs[4])
+                            : p;
+      for (int t = 0; t < kinda; ++t) {
+        const int set = (KIND == 2 && t == 1) ? 2 : t;  // final stage: ain, ta
+        tma_prefetch(&M.aux[d][set], bx, by, bz, c0);
       }
-      pend |= 1u << s;
-    };
+    }
+  };
+  for (int q = 0; q < NSLOT; ++q)
+    if (q <= n) issue(q, q);
+  auto wait = [&](int s) -> bool {  // every thread, in march order
+    const bool ok = mbar_wait(&bars[s], (rs.ph >> s) & 1u, wk.wait_us);
+    if (ok) {  // an expired wait leaves the copy pending for the drain
+      rs.ph ^= 1u << s;
+      rs.pend &= ~(1u << s);
+    }
+    return ok;
+  };
 
-    if (tid == 0)
-      for (int q = 0; q < NSLOT; ++q) issue(it, q, (base + q) & (NSLOT - 1));
-    auto wait = [&](int q) -> bool {  // every thread, in march order
-      const int s = (base + q) & (NSLOT - 1);
-      const bool ok = mbar_wait(&bars[s], (ph >> s) & 1u, wk.wait_us);
-      if (ok) {  // an expired wait leaves the copy pending for the drain
-        ph ^= 1u << s;
-        if (tid == 0) pend &= ~(1u << s);
-      }
-      return ok;
-    };
-
-    Pair e;
-    e.i = i0 + 2 * tx;
-    e.j = j0 + ty;
-    e.ix = e.i + XO;
-    e.iy = e.j + LFD;
-    const bool rowok = e.j < g.nj;  // (tile origins may lie left of the grid)
-    e.m = (rowok && e.i >= 0 && e.i < g.ni ? 1 : 0) | (rowok && e.i + 1 >= 0 && e.i + 1 < g.ni ? 2 : 0);
+  Pair e;
+  e.i = i0 + 2 * tx;
+  e.j = j0 + ty;
+  e.ix = e.i + XO;
+  e.iy = e.j + LFD;
+  e.m = 3;
+  if constexpr (!LEAN) {
+    const bool rowok = e.j >= 0 && e.j < g.nj;  // (tile origins may lie left of the grid)
+    e.m = (rowok && e.i >= 0 && e.i < g.ni ? 1 : 0) |
+          (rowok && e.i + 1 >= 0 && e.i + 1 < g.ni ? 2 : 0);
     auto inx = [&](int i) { return i < g.nabs[0] || i >= g.ni - g.nabs[1]; };
     e.mx = ((e.m & 1) && inx(e.i) ? 1 : 0) | ((e.m & 2) && inx(e.i + 1) ? 2 : 0);
     e.ypml = e.m && (e.j < g.nabs[2] || e.j >= g.nj - g.nabs[3]);
@@ -943,92 +994,164 @@ __global__ void __launch_bounds__(TT, MinCtas<T>::value)
       e.bby = A.b[1][e.iy]; e.iBy = 1.f / e.bby;
       e.apdy = A.apd[1][e.iy]; e.dby = A.db[1][e.iy];
     }
-    // tile-uniform: no x/y PML anywhere in this tile (and B = 1, DB = APD = 0
-    // outside the layers, which the solver checks at upload)
-    const bool tile_int = A.plain_interior && (i0 >= g.nabs[0]) &&
-                          (i0 + CX <= g.ni - g.nabs[1]) && (j0 >= g.nabs[2]) &&
-                          (j0 + TY <= g.nj - g.nabs[3]);
-
-    // register window: w[c][q] = plane (current) + DIR * (q - 3)
-    typename Win<T>::type w[NC][5];
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int q = 0; q < 5; ++q) w[c][q] = Win<T>::zero();
-    auto push_smem = [&](const unsigned char *slot) {
-      const T *plane = reinterpret_cast<const T *>(slot);
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[c][q] = w[c][q + 1];
-        w[c][4] = Win<T>::ld(plane + c * HPL + sc);
-      }
-    };
-    // the three planes behind the chunk come straight from global memory
-    for (int k = 3; k >= 1; --k) {
-      const size_t o = gidx(g, e.ix, e.iy, zf - DIR * k);
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[c][q] = w[c][q + 1];
-        const T *src = static_cast<const T *>(A.in) + (size_t)(C0 + c) * fs + o;
-        w[c][4] = e.m ? Win<T>::ldm(src, e.m) : Win<T>::zero();
-      }
-    }
-    // A wait that expires sets the CTA-wide abort flag; the flag is read only
-    // after a __syncthreads, so every thread leaves the march together.
-    if (wait(0)) push_smem(ring + (size_t)(base & (NSLOT - 1)) * S::BYTES);
-    else abort_flag = 1;
-    __syncthreads();
-
-    size_t c = gidx(g, e.ix, e.iy, zf);
-    float zzn = zz_of(zf);
-#pragma unroll MARCH_UNROLL
-    for (int q = 0; q < n; ++q) {
-      const float zzc = zzn;
-      if (q + 1 < n) zzn = zz_of(zf + DIR * (q + 1));
-      const bool got = wait(q + 1);
-      if (got) push_smem(ring + (size_t)((base + q + 1) & (NSLOT - 1)) * S::BYTES);
-      else abort_flag = 1;
-      if (e.m && got) {
-        const unsigned char *slot = ring + (size_t)((base + q) & (NSLOT - 1)) * S::BYTES;
-        Plane pl;
-        pl.iz = zf + DIR * q;
-        pl.k = pl.iz - LFD;
-        pl.c = c;
-        pl.top = (pl.iz == g.top);
-        pl.near_top = pl.iz >= g.top - 2;
-        pl.zpml = (pl.iz < zlo) || (pl.iz >= zhi);
-        pl.curved = pl.iz >= g.con && !flat;
-        pl.lean = tile_int && !pl.zpml && !pl.near_top;
-        pl.met = met_tile(pl.iz);
-        pl.zz = zzc;
-        const Pw2<T> pw{reinterpret_cast<const T *>(slot + S::U0) + tc,
-                        reinterpret_cast<const T *>(slot + S::U1) + tc,
-                        reinterpret_cast<const float *>(slot + S::COEF) + tc,
-                        reinterpret_cast<const float *>(slot + S::MET) + tc};
-        const T *H = reinterpret_cast<const T *>(slot);
-        if constexpr (PART == PART_VEL)
-          vel_pair<T, X, Y, Z, KIND>(A, e, pl, H, ry, cb, pw, w, rx, rys, rz);
-        else
-          str_pair<T, X, Y, Z, KIND>(A, e, pl, H, ry, cb, pw, w, rx, rys, rz);
-      }
-      // the slot of entry q is free: refill it with stream position
-      // base + q + NSLOT (this item's entry q + 4, or the next item's)
-      __syncthreads();
-      if (abort_flag) break;
-      if (tid == 0 && q + NSLOT <= n) issue(it, q + NSLOT, (base + q) & (NSLOT - 1));
-      c += (DIR > 0) ? g.plane : (size_t)0 - g.plane;
-    }
-    __syncthreads();  // all reads of the ring done before the next item reuses it
-    base += n + 1;
   }
-  if (abort_flag && tid == 0) {
-    if (err) atomicExch(err, 1);
-    // drain: wait (bounded) for copies still in flight before the CTA's
-    // shared memory goes away
-    for (int s = 0; s < NSLOT; ++s)
-      if (pend & (1u << s)) mbar_wait(&bars[s], (ph >> s) & 1u, wk.wait_us);
+
+  // register window: w[c][q] = plane (current) + DIR * (q - 3)
+  typename Win<T>::type w[NC][5];
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int q = 0; q < 5; ++q) w[c][q] = Win<T>::zero();
+  auto push_smem = [&](uint32_t slot) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) w[c][q] = w[c][q + 1];
+      w[c][4] = Win<T>::ld(slot + sc + c * (HPL * (int)sizeof(T)));
+    }
+  };
+  // the three planes behind the chunk come straight from global memory
+  for (int k = 3; k >= 1; --k) {
+    const size_t o = gidx(g, e.ix, e.iy, zf - DIR * k);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) w[c][q] = w[c][q + 1];
+      const T *src = static_cast<const T *>(A.in) + (size_t)(C0 + c) * fs + o;
+      w[c][4] = e.m ? Win<T>::ldm(src, e.m) : Win<T>::zero();
+    }
+  }
+  // A wait that expires sets the CTA-wide abort flag; the flag is read only
+  // after a __syncthreads, so every thread leaves the march together.
+  if (!wait(0)) *abort_flag = 1;
+  push_smem(ring32);
+  __syncthreads();
+
+  size_t c = gidx(g, e.ix, e.iy, zf);
+  float zzn = zz_of(zf);
+  int s = 0;  // slot of entry q
+#pragma unroll 1
+  for (int q = 0; q < n; ++q) {
+    const float zzc = zzn;
+    if (q + 1 < n) zzn = zz_of(zf + DIR * (q + 1));
+    const int s1 = s + 1 == NSLOT ? 0 : s + 1;
+    if (!wait(s1)) *abort_flag = 1;
+    push_smem(ring32 + s1 * S::BYTES);
+    // (after an expired wait the plane is computed from what the slot holds and
+    // the march is left at the barrier; made to depend on the wait's outcome,
+    // this branch was never taken in builds under register pressure)
+    int mask = e.m;
+    if constexpr (!LEAN) asm volatile("" : "+r"(mask));
+    if (mask) {
+      const uint32_t slot = ring32 + s * S::BYTES;
+      Plane pl;
+      pl.iz = zf + DIR * q;
+      pl.k = pl.iz - LFD;
+      pl.c = c;
+      pl.top = (pl.iz == g.top);
+      pl.near_top = pl.iz >= g.top - 2;
+      pl.zpml = (pl.iz < zlo) || (pl.iz >= zhi);
+      pl.curved = pl.iz >= g.con && !flat;
+      pl.met = met_tile(pl.iz);
+      pl.zz = zzc;
+      const Pw2<T> pw{slot + S::U0 + tc * (int)sizeof(T), slot + S::U1 + tc * (int)sizeof(T),
+                      slot + S::COEF + tc * 4, slot + S::MET + tc * 4};
+      const uint32_t hp = slot + sc;
+      if constexpr (PART == PART_VEL)
+        vel_pair<T, X, Y, Z, KIND, LEAN>(A, e, pl, hp, pw, w, rh);
+      else
+        str_pair<T, X, Y, Z, KIND, LEAN>(A, e, pl, hp, pw, w, rh);
+    }
+    // the slot of entry q is free: refill it with entry q + NSLOT
+    __syncthreads();
+    if (*abort_flag) return;
+    if (q + NSLOT <= n) issue(q + NSLOT, s);
+    s = s1;
+    c += (DIR > 0) ? g.plane : (size_t)0 - g.plane;
+  }
+}
+
+// A persistent grid over one part of the general items of a stage, or over
+// both parts of the lean ones: there a tile's velocity and stress items follow
+// one another in the list, so the two run side by side and share in L2 what
+// both read.
+template <typename T, int X, int Y, int Z, int KIND, bool B, int LIST>
+__global__ void __launch_bounds__(TT, (Ring<T, LIST>::CTAS))
+    pair_kernel(const __grid_constant__ Maps maps_v, const __grid_constant__ Maps maps_s,
+                const StageArgs a, const Work wk, int *err) {
+  using R = Ring<T, LIST>;
+  constexpr bool LEAN = R::LEAN;
+  constexpr int NSLOT = R::NSLOT;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  // align the ring on the shared-window address itself
+  unsigned char *sbase = smem_raw + ((128u - (su32(smem_raw) & 127u)) & 127u);
+  unsigned char *ring = sbase;  // NSLOT slots
+  uint64_t *bars = reinterpret_cast<uint64_t *>(sbase + (size_t)NSLOT * R::BYTES);
+  __shared__ volatile int abort_flag;
+  __shared__ volatile int s_next;
+  const int tid = threadIdx.y * TX + threadIdx.x;
+
+  if (tid == 0) {
+    abort_flag = 0;
+    const bool aligned = ((su32(bars) & 7u) == 0) && ((su32(ring) & 127u) == 0);
+    if (!aligned) {
+      abort_flag = 1;
+      if (err) atomicExch(err, 2);
+    } else {
+      for (int s = 0; s < NSLOT; ++s) mbar_init(&bars[s], NWARP);
+      fence_mbar_init();
+    }
+  }
+  __syncthreads();
+  RingState rs;
+  int *const counter = wk.counter + 2 * LIST;
+  if (!abort_flag) {
+    for (;;) {
+      // the next item, taken only when this CTA is free (a CTA never holds a
+      // claim on work while it is still busy)
+      if (tid == 0) s_next = atomicAdd(counter, 1);
+      __syncthreads();
+      const int cur = s_next;
+      if (cur >= wk.nitems[LEAN]) break;  // CTA-uniform
+      const int4 it4 = wk.items[LEAN][cur];
+      const int part = LEAN ? it4.w & 1 : LIST, model = B ? it4.w >> 1 : 0;
+      // a batched launch reads the item's model's stage arguments in place
+      // (global memory, read-only during the launch).  Copied per item into a
+      // __shared__ StageArgs and read from there, the 16-bit batched stages
+      // behaved as if every component scale were zero (FP32, whose kernels
+      // never read the scales, was unaffected); read through a pointer to the
+      // copy hidden from the compiler they were correct but 15% slower than
+      // in place.
+      const StageArgs &A = B ? wk.bargs[model] : a;
+      const bool aux_on[3] = {B ? A.ain[0] != nullptr : wk.has_aux[0] != 0,
+                              B ? A.ain[1] != nullptr : wk.has_aux[1] != 0,
+                              B ? A.ain[2] != nullptr : wk.has_aux[2] != 0};
+      const int4 it = make_int4(it4.x, it4.y, it4.z & 0xffff, it4.z >> 16);
+      if (LIST == GEN_VEL || (LEAN && part == PART_VEL))
+        march<T, PART_VEL, X, Y, Z, KIND, LEAN>(A, B ? wk.bmaps[model] : maps_v, wk, aux_on, it,
+                                                cur == 0, ring, bars, rs, &abort_flag);
+      else if (LIST != GEN_VEL)
+        march<T, PART_STR, X, Y, Z, KIND, LEAN>(
+            A, B ? wk.bmaps[wk.nmodels + model] : maps_s, wk, aux_on, it, false, ring, bars, rs,
+            &abort_flag);
+      __syncthreads();  // all reads of the ring done before the next item reuses it
+      if (abort_flag) break;
+    }
+    if (abort_flag && tid == 0) {
+      if (err) atomicExch(err, 1);
+      // drain: wait (bounded) for copies still in flight before the CTA's
+      // shared memory goes away
+      for (int s = 0; s < NSLOT; ++s)
+        if (rs.pend & (1u << s)) mbar_wait(&bars[s], (rs.ph >> s) & 1u, wk.wait_us);
+    }
+  }
+  // the last CTA to finish resets the counters for the next launch
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(counter + 1, 1) == (int)gridDim.x - 1) {
+      counter[0] = 0;
+      counter[1] = 0;
+    }
   }
 }
 
@@ -1046,10 +1169,11 @@ struct ModelMaps {
 struct Plan {
   std::vector<ModelMaps> mm;   // one per model
   std::vector<Geom> geoms;
+  std::vector<char> plain;     // per model: StageArgs::plain_interior
   Work wk;
   int elem;                    // storage element type of the field sets
   int zchunk;                  // planes of the (first model's) interior z-chunks
-  int grid[2];
+  int grid[NLIST];             // CTAs per launch (0: no items)
   WorkParams params;
   int nmodels = 0;             // 0: single-model plan; else a batch of nmodels
   StageArgs *d_bargs = nullptr;  // batch: [pattern * 4 + stage][model]
@@ -1058,89 +1182,81 @@ struct Plan {
 
 // a: the single model's stage arguments (X, Y, Z and the stage kind come
 // from it in every case); a batched launch (B) takes each model's arguments
-// and maps from pl.wk instead
-template <typename T, int PART, int X, int Y, int Z, int KIND, bool B>
-void launch_t(const Plan &pl, const Maps &m, const StageArgs &a, const Work &wk, int *err,
+// and maps from wk instead
+template <typename T, int X, int Y, int Z, int KIND, bool B, int LIST>
+void launch_t(const Plan &pl, const Maps *m, const StageArgs &a, const Work &wk, int *err,
               cudaStream_t s) {
-  pair_kernel<T, PART, X, Y, Z, KIND, B>
-      <<<pl.grid[PART], dim3(TX, TY, 1), Slot<T, PART>::SMEM, s>>>(m, a, wk, err);
+  pair_kernel<T, X, Y, Z, KIND, B, LIST>
+      <<<pl.grid[LIST], dim3(TX, TY, 1), Ring<T, LIST>::SMEM, s>>>(m[0], m[1], a, wk, err);
 }
 
-template <typename T, int PART, int KIND, bool B = false>
-void launch_dirs(const Plan &pl, const Maps &m, const StageArgs &a, const Work &wk, int *err,
+template <typename T, int KIND, bool B, int LIST>
+void launch_dirs(const Plan &pl, const Maps *m, const StageArgs &a, const Work &wk, int *err,
                  cudaStream_t s) {
   const int code = (a.X > 0 ? 4 : 0) + (a.Y > 0 ? 2 : 0) + (a.Z > 0 ? 1 : 0);
   switch (code) {
-    case 0: launch_t<T, PART, -1, -1, -1, KIND, B>(pl, m, a, wk, err, s); break;
-    case 1: launch_t<T, PART, -1, -1, 1, KIND, B>(pl, m, a, wk, err, s); break;
-    case 2: launch_t<T, PART, -1, 1, -1, KIND, B>(pl, m, a, wk, err, s); break;
-    case 3: launch_t<T, PART, -1, 1, 1, KIND, B>(pl, m, a, wk, err, s); break;
-    case 4: launch_t<T, PART, 1, -1, -1, KIND, B>(pl, m, a, wk, err, s); break;
-    case 5: launch_t<T, PART, 1, -1, 1, KIND, B>(pl, m, a, wk, err, s); break;
-    case 6: launch_t<T, PART, 1, 1, -1, KIND, B>(pl, m, a, wk, err, s); break;
-    default: launch_t<T, PART, 1, 1, 1, KIND, B>(pl, m, a, wk, err, s); break;
+    case 0: launch_t<T, -1, -1, -1, KIND, B, LIST>(pl, m, a, wk, err, s); break;
+    case 1: launch_t<T, -1, -1, 1, KIND, B, LIST>(pl, m, a, wk, err, s); break;
+    case 2: launch_t<T, -1, 1, -1, KIND, B, LIST>(pl, m, a, wk, err, s); break;
+    case 3: launch_t<T, -1, 1, 1, KIND, B, LIST>(pl, m, a, wk, err, s); break;
+    case 4: launch_t<T, 1, -1, -1, KIND, B, LIST>(pl, m, a, wk, err, s); break;
+    case 5: launch_t<T, 1, -1, 1, KIND, B, LIST>(pl, m, a, wk, err, s); break;
+    case 6: launch_t<T, 1, 1, -1, KIND, B, LIST>(pl, m, a, wk, err, s); break;
+    default: launch_t<T, 1, 1, 1, KIND, B, LIST>(pl, m, a, wk, err, s); break;
   }
 }
 
-template <typename T, int PART, int KIND, bool B = false>
+template <typename T, int KIND, bool B, int LIST>
 void set_attrs() {
   auto set = [](const void *f) {
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Slot<T, PART>::SMEM);
+                         (int)Ring<T, LIST>::SMEM);
   };
-  set((const void *)pair_kernel<T, PART, -1, -1, -1, KIND, B>);
-  set((const void *)pair_kernel<T, PART, -1, -1, 1, KIND, B>);
-  set((const void *)pair_kernel<T, PART, -1, 1, -1, KIND, B>);
-  set((const void *)pair_kernel<T, PART, -1, 1, 1, KIND, B>);
-  set((const void *)pair_kernel<T, PART, 1, -1, -1, KIND, B>);
-  set((const void *)pair_kernel<T, PART, 1, -1, 1, KIND, B>);
-  set((const void *)pair_kernel<T, PART, 1, 1, -1, KIND, B>);
-  set((const void *)pair_kernel<T, PART, 1, 1, 1, KIND, B>);
+  set((const void *)pair_kernel<T, -1, -1, -1, KIND, B, LIST>);
+  set((const void *)pair_kernel<T, -1, -1, 1, KIND, B, LIST>);
+  set((const void *)pair_kernel<T, -1, 1, -1, KIND, B, LIST>);
+  set((const void *)pair_kernel<T, -1, 1, 1, KIND, B, LIST>);
+  set((const void *)pair_kernel<T, 1, -1, -1, KIND, B, LIST>);
+  set((const void *)pair_kernel<T, 1, -1, 1, KIND, B, LIST>);
+  set((const void *)pair_kernel<T, 1, 1, -1, KIND, B, LIST>);
+  set((const void *)pair_kernel<T, 1, 1, 1, KIND, B, LIST>);
 }
 
-template <typename T, int PART, bool B = false>
+template <typename T, bool B, int LIST>
 int resident_ctas() {
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, pair_kernel<T, PART, 1, 1, 1, 1, B>, TT,
-                                                Slot<T, PART>::SMEM);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, pair_kernel<T, 1, 1, 1, 1, B, LIST>, TT,
+                                                Ring<T, LIST>::SMEM);
   if (per < 1) per = 1;
   if (sms < 1) sms = 1;
   return per * sms;
 }
 
-// per-(storage, part, kind) entry points, one translation unit each
-// (pair_{f,h,b}{v,s}{0,1,2}.cu; f: FP32, h: FP16, b: BF16 storage), each
-// with its batched kernels (suffix _b)
-#define CGFD_PAIR_DECL(E, P, K)                                                          \
-  void launch_##E##P##K(const Plan &pl, const Maps &m, const StageArgs &a, int *err,   \
-                        cudaStream_t s);                                                \
-  void attrs_##E##P##K();
-#define CGFD_PAIR_DECL_B(E, P, K)                                                        \
-  void launch_##E##P##K##_b(const Plan &pl, const StageArgs &a, const Work &wk, int *err, \
-                            cudaStream_t s);                                            \
-  void attrs_##E##P##K##_b();
-#define CGFD_PAIR_DECL_E(E)                                                   \
-  CGFD_PAIR_DECL(E, v, 0) CGFD_PAIR_DECL(E, v, 1) CGFD_PAIR_DECL(E, v, 2)     \
-  CGFD_PAIR_DECL(E, s, 0) CGFD_PAIR_DECL(E, s, 1) CGFD_PAIR_DECL(E, s, 2)     \
-  int resident_##E##v();                                                      \
-  int resident_##E##s();
-CGFD_PAIR_DECL_E(f)
-CGFD_PAIR_DECL_E(h)
-CGFD_PAIR_DECL_E(b)
-#define CGFD_PAIR_DECL_BE(E)                                                         \
-  CGFD_PAIR_DECL_B(E, v, 0) CGFD_PAIR_DECL_B(E, v, 1) CGFD_PAIR_DECL_B(E, v, 2)          \
-  CGFD_PAIR_DECL_B(E, s, 0) CGFD_PAIR_DECL_B(E, s, 1) CGFD_PAIR_DECL_B(E, s, 2)          \
-  int resident_##E##v_b();                                                            \
-  int resident_##E##s_b();
-CGFD_PAIR_DECL_BE(f)
-CGFD_PAIR_DECL_BE(h)
-CGFD_PAIR_DECL_BE(b)
-#undef CGFD_PAIR_DECL_BE
-#undef CGFD_PAIR_DECL_B
-#undef CGFD_PAIR_DECL_E
+// Entry points per storage type (f: FP32, h: FP16, b: BF16), RK stage kind
+// and launch (v, s: general velocity, stress; l: lean), one translation unit each (pair_*.cu).
+typedef void (*LaunchFn)(const Plan &, const Maps *, const StageArgs &, const Work &, int *,
+                         cudaStream_t);
+struct Entry {
+  LaunchFn launch[2];     // [batched]
+  void (*attrs)();        // both forms
+  int (*resident[2])();   // [batched] CTAs resident on the device
+};
+#define CGFD_PAIR_DECL(E) \
+  Entry entry_##E##0v(), entry_##E##1v(), entry_##E##2v(), entry_##E##0s(), entry_##E##1s(), \
+      entry_##E##2s(), entry_##E##0l(), entry_##E##1l(), entry_##E##2l();
+CGFD_PAIR_DECL(f)
+CGFD_PAIR_DECL(h)
+CGFD_PAIR_DECL(b)
 #undef CGFD_PAIR_DECL
+template <typename T, int KIND, int LIST>
+Entry make_entry() {
+  return Entry{{launch_dirs<T, KIND, false, LIST>, launch_dirs<T, KIND, true, LIST>},
+               [] { set_attrs<T, KIND, false, LIST>(); set_attrs<T, KIND, true, LIST>(); },
+               {[]() -> int { if constexpr (KIND == 1) return resident_ctas<T, false, LIST>(); else return 0; },
+                []() -> int { if constexpr (KIND == 1) return resident_ctas<T, true, LIST>(); else return 0; }}};
+}
 
 }  // namespace pair
 }  // namespace cgfd
