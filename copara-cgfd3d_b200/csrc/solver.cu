@@ -376,6 +376,10 @@ struct cgfd_solver {
   Geom g{};
   cudaStream_t st = nullptr;
   SideStream side{};  // the launches of a stage beside one another
+  // device staging of uploads, downloads and snapshots (one array at a time,
+  // on the solver's stream), kept between calls up to STAGE_KEEP bytes
+  float *stage = nullptr;
+  size_t stage_cap = 0;
   // host-to-device upload staging: the copy events of the two pinned chunks
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
   std::string err;
@@ -508,6 +512,8 @@ int arg_fail(cgfd_solver *h, const char *what) {
   } while (0)
 
 void free_all(cgfd_solver *h) {
+  cudaFree(h->stage);
+  h->stage = nullptr;
   if (h->plan) {
     if (h->d.kernel == CGFD_KERNEL_FUSED) pair_destroy_plan(h->plan);
     else fused_destroy_plan(h->plan);
@@ -533,6 +539,41 @@ void free_all(cgfd_solver *h) {
   }
 }
 
+// Device staging of n floats on the solver's stream.  cudaMalloc and cudaFree
+// per call cost about 0.6 ms of a snapshot (both synchronise the device), more
+// than ten steps of a small model; buffers up to STAGE_KEEP stay with the
+// solver (grown, never shrunk, freed with it), larger ones live for the call.
+constexpr size_t STAGE_KEEP = 64u << 20;
+struct Stage {
+  cgfd_solver *h;
+  float *p = nullptr;
+  bool own = false;
+  Stage(cgfd_solver *hh, size_t n) : h(hh) {
+    const size_t b = n * sizeof(float);
+    if (b > STAGE_KEEP) {
+      own = cudaMalloc(&p, b) == cudaSuccess;
+      if (!own) p = nullptr, cudaGetLastError();
+      return;
+    }
+    if (b > h->stage_cap) {
+      cudaFree(h->stage);
+      h->stage = nullptr;
+      h->stage_cap = 0;
+      if (cudaMalloc(&h->stage, b) != cudaSuccess) {
+        h->stage = nullptr;
+        cudaGetLastError();
+        return;
+      }
+      h->stage_cap = b;
+    }
+    p = h->stage;
+  }
+  Stage(const Stage &) = delete;
+  ~Stage() {
+    if (own) cudaFree(p);
+  }
+};
+
 long ref_n(const cgfd_solver *h) {
   return (long)(h->d.ni + 6) * (h->d.nj + 6) * (h->d.nk + 6);
 }
@@ -542,8 +583,9 @@ long ref_n(const cgfd_solver *h) {
 int upload_ref(cgfd_solver *h, const float *host, void *dst, int elem = ELEM_F32,
                float isc = 1.f) {
   const long n = ref_n(h);
-  float *tmp = nullptr;
-  CK(h, cudaMalloc(&tmp, n * sizeof(float)));
+  Stage stage(h, n);
+  float *const tmp = stage.p;
+  if (!tmp) return cuda_fail(h, cudaErrorMemoryAllocation, "upload");
   cudaError_t e = cudaMemcpyAsync(tmp, host, n * sizeof(float), cudaMemcpyHostToDevice, h->st);
   if (e == cudaSuccess) {
     const int nx = h->d.ni + 6, ny = h->d.nj + 6, nz = h->d.nk + 6;
@@ -557,7 +599,6 @@ int upload_ref(cgfd_solver *h, const float *host, void *dst, int elem = ELEM_F32
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-  cudaFree(tmp);
   if (e != cudaSuccess) return cuda_fail(h, e, "upload");
   return CGFD_OK;
 }
@@ -601,8 +642,9 @@ int upload_fields(cgfd_solver *h, int count, Fill &&fill, float *const *dst) {
       CK(h, cudaHostAlloc((void **)&g_pin[q], PIN_CHUNK * sizeof(float), cudaHostAllocPortable));
     if (!h->pin_ev[q]) CK(h, cudaEventCreateWithFlags(&h->pin_ev[q], cudaEventDisableTiming));
   }
-  float *tmp = nullptr;
-  CK(h, cudaMalloc(&tmp, n * sizeof(float)));
+  Stage stage(h, n);
+  float *const tmp = stage.p;
+  if (!tmp) return cuda_fail(h, cudaErrorMemoryAllocation, "upload");
   const int nx = h->d.ni + 6, ny = h->d.nj + 6, nz = h->d.nk + 6;
   cudaError_t e = cudaSuccess;
   int c = 0;
@@ -622,7 +664,6 @@ int upload_fields(cgfd_solver *h, int count, Fill &&fill, float *const *dst) {
     }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-  cudaFree(tmp);
   if (e != cudaSuccess) return cuda_fail(h, e, "upload");
   return CGFD_OK;
 }
@@ -630,8 +671,9 @@ int upload_fields(cgfd_solver *h, int count, Fill &&fill, float *const *dst) {
 int download_ref(cgfd_solver *h, const void *src, float *host, int elem = ELEM_F32,
                  float sc = 1.f) {
   const long n = ref_n(h);
-  float *tmp = nullptr;
-  CK(h, cudaMalloc(&tmp, n * sizeof(float)));
+  Stage stage(h, n);
+  float *const tmp = stage.p;
+  if (!tmp) return cuda_fail(h, cudaErrorMemoryAllocation, "download");
   const int nx = h->d.ni + 6, ny = h->d.nj + 6, nz = h->d.nk + 6;
   if (elem == ELEM_F16)
     to_reference_kernel<<<592, 256, 0, h->st>>>((const __half *)src, tmp, h->g, nx, ny, nz, sc);
@@ -644,7 +686,6 @@ int download_ref(cgfd_solver *h, const void *src, float *host, int elem = ELEM_F
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(host, tmp, n * sizeof(float), cudaMemcpyDeviceToHost, h->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-  cudaFree(tmp);
   if (e != cudaSuccess) return cuda_fail(h, e, "download");
   return CGFD_OK;
 }
@@ -2569,8 +2610,9 @@ int cgfd_get_snapshot(cgfd_solver *h, int set, const int *start, const int *coun
   // 16-bit storage keeps tW - FW: gather FW too and add it back
   const bool add_fw = set == CGFD_SET_TW && h->elem != ELEM_F32;
   const int parts = add_fw ? 2 : 1;
-  float *tmp = nullptr;
-  CK(h, cudaMalloc(&tmp, parts * n * sizeof(float)));
+  Stage stage(h, parts * n);
+  float *const tmp = stage.p;
+  if (!tmp) return cuda_fail(h, cudaErrorMemoryAllocation, "snapshot");
   ScaleSet sc;
   for (int c = 0; c < NCOMP; ++c) sc.sc[c] = std::ldexp(1.f, h->sexp[c]);
   const int3 st3 = make_int3(start[0], start[1], start[2]);
@@ -2596,7 +2638,6 @@ int cgfd_get_snapshot(cgfd_solver *h, int set, const int *start, const int *coun
   if (e == cudaSuccess && add_fw)
     e = cudaMemcpyAsync(fw.data(), tmp + n, n * sizeof(float), cudaMemcpyDeviceToHost, h->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-  cudaFree(tmp);
   if (e != cudaSuccess) return cuda_fail(h, e, "snapshot");
   for (size_t t = 0; t < fw.size(); ++t) out[t] += fw[t];
   return CGFD_OK;
