@@ -40,13 +40,23 @@
 //
 // Training kernel: for samples (x, t) of normalised features and target
 // corrections, the mean squared error over samples and its gradient with
-// respect to every parameter.  A block takes chunks of 128 samples: one
-// thread per sample runs the forward and backward pass (FP32) and leaves
-// the inputs, activations and back-propagated errors in shared memory; then
-// every thread sums, over the chunk's samples, the products for the
-// parameters it owns (a block-level reduction, no atomics), carrying the
-// sums across the block's chunks; per-block partial gradients are summed in
-// block order by a second kernel, so the result does not depend on timing.
+// respect to every parameter.  A block takes chunks of 128 samples; two
+// threads per sample run the forward and backward pass (FP32), each over half
+// of a layer's units in groups of eight, and leave the inputs, activations and
+// back-propagated errors in shared memory; then every thread sums, over the
+// chunk's samples, the products of a small tile of each weight matrix (a
+// block-level reduction, no atomics), carrying the sums across the block's
+// chunks; per-block partial gradients are summed in block order by a second
+// kernel, so the result does not depend on timing.
+//
+// Shared memory (the activations of 128 samples and the weights, 210 KB)
+// leaves one block per SM, so what bounds the kernel is the latency of its
+// dependent chains: one thread per sample with one running sum at a time, and
+// one dot product at a time in the gradient, made a call with 20000 samples take
+// 726 us (copies included);
+// eight sums per thread that share each activation load, weights stored so
+// that eight of them are two 128-bit broadcast loads, and 4 x 4 gradient tiles
+// (eight loads for sixteen products) make it 422 us (111 us in this kernel).
 #include "../../include/cgfd.h"
 #include "abi_guard.h"
 #include "cgfd_internal.cuh"
@@ -356,119 +366,206 @@ __global__ void features_kernel(const T *__restrict__ fw, size_t fs, ScaleSet sc
 }
 
 // ------------------------------- training ---------------------------------
-constexpr int GB = 128;       // samples per chunk = threads per block
+constexpr int GB = 128;       // samples per chunk
+constexpr int GT = 2 * GB;    // threads per block
 constexpr int LDS = GB + 1;   // row stride of the per-chunk arrays (bank spread)
-constexpr int PER_T = (NPAR + GB - 1) / GB;  // parameters owned per thread
-// shared memory: FP32 parameters, then [row][sample] arrays of the chunk
+// weights in shared memory, rows of the units that a thread computes together
+// (16-byte aligned): [k][unit] for the forward pass, [unit][k] for the backward
+constexpr int LD3 = 12;       // outputs padded
+struct GSmem {
+  float w1t[NIN * NH], w2t[NH * NH], w2[NH * NH], w3[NOUT * NH], w3t[NH * LD3];
+  float b1[NH], b2[NH], b3[LD3];
+};
+// [row][sample] arrays of the chunk
 constexpr int R_X = 0, R_H1 = R_X + NIN, R_H2 = R_H1 + NH, R_DY = R_H2 + NH;
 constexpr int R_D2 = R_DY + NOUT, R_D1 = R_D2 + NH, NROWS = R_D1 + NH;
-constexpr size_t GRAD_SMEM = (NPAR + (size_t)NROWS * LDS) * sizeof(float);
+constexpr size_t GRAD_SMEM = sizeof(GSmem) + (size_t)NROWS * LDS * sizeof(float);
+static_assert(sizeof(GSmem) % 16 == 0 && GRAD_SMEM <= 227 * 1024, "gradient kernel");
 
-// the sum over the chunk of (row a) * (row b), or of row a (b < 0)
-__device__ __forceinline__ float row_dot(const float *ch, int a, int b) {
-  const float *pa = ch + a * LDS;
-  float s = 0.f;
-  if (b < 0) {
-    for (int k = 0; k < GB; ++k) s += pa[k];
-  } else {
-    const float *pb = ch + b * LDS;
-    for (int k = 0; k < GB; ++k) s = fmaf(pa[k], pb[k], s);
+// a[0..7] += w[k][u0 .. u0+7] * x[k] over k, in order; w: rows of LD values,
+// x: rows of the chunk at this thread's sample
+template <int K, int LD>
+__device__ __forceinline__ void units8(const float *w, int u0, const float *x, float (&a)[8]) {
+#pragma unroll 4
+  for (int k = 0; k < K; ++k) {
+    const float4 p = *reinterpret_cast<const float4 *>(w + k * LD + u0);
+    const float4 q = *reinterpret_cast<const float4 *>(w + k * LD + u0 + 4);
+    const float v = x[k * LDS];
+    a[0] = fmaf(p.x, v, a[0]); a[1] = fmaf(p.y, v, a[1]);
+    a[2] = fmaf(p.z, v, a[2]); a[3] = fmaf(p.w, v, a[3]);
+    a[4] = fmaf(q.x, v, a[4]); a[5] = fmaf(q.y, v, a[5]);
+    a[6] = fmaf(q.z, v, a[6]); a[7] = fmaf(q.w, v, a[7]);
   }
-  return s;
 }
-// rows whose product over samples is parameter p's gradient
-__device__ __forceinline__ void param_rows(int p, int *a, int *b) {
-  if (p < OB1) { *a = R_D1 + (p - OW1) / NIN; *b = R_X + (p - OW1) % NIN; }
-  else if (p < OW2) { *a = R_D1 + (p - OB1); *b = -1; }
-  else if (p < OB2) { *a = R_D2 + (p - OW2) / NH; *b = R_H1 + (p - OW2) % NH; }
-  else if (p < OW3) { *a = R_D2 + (p - OB2); *b = -1; }
-  else if (p < OB3) { *a = R_DY + (p - OW3) / NH; *b = R_H2 + (p - OW3) % NH; }
-  else { *a = R_DY + (p - OB3); *b = -1; }
+// acc[i][j] += the sum over the chunk's samples of row a + SI i times row
+// b + SJ j
+template <int NI, int NJ, int SI, int SJ>
+__device__ __forceinline__ void tile_dot(const float *ch, int a, int b, float (&acc)[NI][NJ]) {
+  const float *pa = ch + a * LDS, *pb = ch + b * LDS;
+  float s[NI][NJ];
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) s[i][j] = 0.f;
+#pragma unroll 2
+  for (int k = 0; k < GB; ++k) {
+    float u[NI], v[NJ];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) u[i] = pa[i * SI * LDS + k];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) v[j] = pb[j * SJ * LDS + k];
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) s[i][j] = fmaf(u[i], v[j], s[i][j]);
+  }
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) acc[i][j] += s[i][j];
 }
 
-__global__ void __launch_bounds__(GB)
+__global__ void __launch_bounds__(GT)
     grad_kernel(const __half *__restrict__ w, const float *__restrict__ xs,
                 const float *__restrict__ ts, int n, float *__restrict__ partial) {
   extern __shared__ __align__(16) unsigned char gsm[];
-  float *sw = reinterpret_cast<float *>(gsm);  // NPAR parameters (FP32)
-  float *ch = sw + NPAR;                       // the chunk's rows
-  for (int q = threadIdx.x; q < NPAR; q += GB) sw[q] = __half2float(w[q]);
+  GSmem &W = *reinterpret_cast<GSmem *>(gsm);
+  float *ch = reinterpret_cast<float *>(gsm + sizeof(GSmem));  // the chunk's rows
+  const int tid = threadIdx.x;
+  auto wt = [&](int q) { return __half2float(w[q]); };
+  for (int q = tid; q < NH * NIN; q += GT) W.w1t[(q % NIN) * NH + q / NIN] = wt(OW1 + q);
+  for (int q = tid; q < NH * NH; q += GT) {
+    const float v = wt(OW2 + q);
+    W.w2[q] = v;
+    W.w2t[(q % NH) * NH + q / NH] = v;
+  }
+  for (int q = tid; q < NOUT * NH; q += GT) {
+    const float v = wt(OW3 + q);
+    W.w3[q] = v;
+    W.w3t[(q % NH) * LD3 + q / NH] = v;
+  }
+  for (int q = tid; q < NH; q += GT) {
+    W.b1[q] = wt(OB1 + q);
+    W.b2[q] = wt(OB2 + q);
+  }
+  for (int q = tid; q < NOUT; q += GT) W.b3[q] = wt(OB3 + q);
   __syncthreads();
-  const int s = threadIdx.x;
+  const int s = tid & (GB - 1), h = tid / GB, u0 = h * (NH / 2);
   const float inv_n = 1.f / (float)n;
-  float acc[PER_T];
-#pragma unroll
-  for (int e = 0; e < PER_T; ++e) acc[e] = 0.f;
-  float lsum = 0.f;
+  // this thread's gradient tiles: W2 rows ti + 16 i, columns tj + 16 j; W1
+  // columns tj + 15 j (tj < 15); W3 rows tk + 3 i, column tl (tk < 3); a bias
+  const int ti = tid >> 4, tj = tid & 15, tk = tid >> 6, tl = tid & 63;
+  const int brow = tid < NH ? R_D1 + tid : tid < 2 * NH ? R_D2 + tid - NH : R_DY + tid - 2 * NH;
+  float g2[4][4] = {}, g1[4][3] = {}, g3[3][1] = {}, gb = 0.f, lsum = 0.f;
   for (int c0 = blockIdx.x * GB; c0 < n; c0 += gridDim.x * GB) {
     const int sample = c0 + s;
     const bool live = sample < n;
-    // forward and backward of this thread's sample, into the chunk's rows
-    for (int k = 0; k < NIN; ++k) ch[(R_X + k) * LDS + s] = live ? xs[(size_t)sample * NIN + k] : 0.f;
-    for (int o = 0; o < NH; ++o) {
-      float a = sw[OB1 + o];
-      for (int k = 0; k < NIN; ++k) a = fmaf(sw[OW1 + o * NIN + k], ch[(R_X + k) * LDS + s], a);
-      ch[(R_H1 + o) * LDS + s] = silu(a);
-      ch[(R_D1 + o) * LDS + s] = dsilu(a);  // dL/da1 after the backward pass
+    float *const col = ch + s;  // this thread's sample
+    // inputs (the block's threads read them in memory order)
+    for (int q = tid; q < GB * NIN; q += GT) {
+      const int r = q / NIN;
+      ch[(R_X + q % NIN) * LDS + r] = c0 + r < n ? xs[(size_t)c0 * NIN + q] : 0.f;
     }
-    for (int o = 0; o < NH; ++o) {
-      float a = sw[OB2 + o];
-      for (int k = 0; k < NH; ++k) a = fmaf(sw[OW2 + o * NH + k], ch[(R_H1 + k) * LDS + s], a);
-      ch[(R_H2 + o) * LDS + s] = silu(a);
-      ch[(R_D2 + o) * LDS + s] = dsilu(a);  // dL/da2 after the backward pass
+    __syncthreads();
+    // silu and its derivative (dL/da after the backward pass) of eight units
+    auto activate = [&](const float (&a)[8], int rh, int rd, int o) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        col[(rh + o + e) * LDS] = silu(a[e]);
+        col[(rd + o + e) * LDS] = dsilu(a[e]);
+      }
+    };
+    for (int o = u0; o < u0 + NH / 2; o += 8) {
+      float a[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] = W.b1[o + e];
+      units8<NIN, NH>(W.w1t, o, col + R_X * LDS, a);
+      activate(a, R_H1, R_D1, o);
     }
-    for (int c = 0; c < NOUT; ++c) {
-      float y = sw[OB3 + c];
-      for (int k = 0; k < NH; ++k) y = fmaf(sw[OW3 + c * NH + k], ch[(R_H2 + k) * LDS + s], y);
-      const float e = live ? y - ts[(size_t)sample * NOUT + c] : 0.f;
-      lsum += e * e;
-      ch[(R_DY + c) * LDS + s] = 2.f * e * inv_n;
+    __syncthreads();
+    for (int o = u0; o < u0 + NH / 2; o += 8) {
+      float a[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] = W.b2[o + e];
+      units8<NH, NH>(W.w2t, o, col + R_H1 * LDS, a);
+      activate(a, R_H2, R_D2, o);
     }
-    for (int q = 0; q < NH; ++q) {  // dL/da2
-      float d = 0.f;
-      for (int c = 0; c < NOUT; ++c) d = fmaf(sw[OW3 + c * NH + q], ch[(R_DY + c) * LDS + s], d);
-      ch[(R_D2 + q) * LDS + s] *= d;
+    __syncthreads();
+    if (h == 0) {
+      float y[NOUT];
+#pragma unroll
+      for (int c = 0; c < NOUT; ++c) y[c] = W.b3[c];
+      for (int k = 0; k < NH; ++k) {
+        const float v = col[(R_H2 + k) * LDS];
+#pragma unroll
+        for (int c = 0; c < NOUT; ++c) y[c] = fmaf(W.w3t[k * LD3 + c], v, y[c]);
+      }
+#pragma unroll
+      for (int c = 0; c < NOUT; ++c) {
+        const float e = live ? y[c] - ts[(size_t)sample * NOUT + c] : 0.f;
+        lsum += e * e;
+        col[(R_DY + c) * LDS] = 2.f * e * inv_n;
+      }
     }
-    for (int q = 0; q < NH; ++q) {  // dL/da1
-      float d = 0.f;
-      for (int o = 0; o < NH; ++o) d = fmaf(sw[OW2 + o * NH + q], ch[(R_D2 + o) * LDS + s], d);
-      ch[(R_D1 + q) * LDS + s] *= d;
+    __syncthreads();
+    for (int o = u0; o < u0 + NH / 2; o += 8) {  // dL/da2
+      float a[8] = {};
+      units8<NOUT, NH>(W.w3, o, col + R_DY * LDS, a);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) col[(R_D2 + o + e) * LDS] *= a[e];
+    }
+    __syncthreads();
+    for (int o = u0; o < u0 + NH / 2; o += 8) {  // dL/da1
+      float a[8] = {};
+      units8<NH, NH>(W.w2, o, col + R_D2 * LDS, a);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) col[(R_D1 + o + e) * LDS] *= a[e];
     }
     __syncthreads();
     // the chunk's contribution to this thread's parameters
-#pragma unroll
-    for (int e = 0; e < PER_T; ++e) {
-      const int p = threadIdx.x + e * GB;
-      if (p < NPAR) {
-        int a, b;
-        param_rows(p, &a, &b);
-        acc[e] += row_dot(ch, a, b);
-      }
+    tile_dot<4, 4, 16, 16>(ch, R_D2 + ti, R_H1 + tj, g2);
+    if (tj < 15) tile_dot<4, 3, 16, 15>(ch, R_D1 + ti, R_X + tj, g1);
+    if (tk < 3) tile_dot<3, 1, 3, 1>(ch, R_DY + tk, R_H2 + tl, g3);
+    if (tid < 2 * NH + NOUT) {
+      float v = 0.f;
+      for (int k = 0; k < GB; ++k) v += ch[brow * LDS + k];
+      gb += v;
     }
     __syncthreads();  // the rows are rewritten by the next chunk
   }
   float *out = partial + (size_t)blockIdx.x * (NPAR + 1);
 #pragma unroll
-  for (int e = 0; e < PER_T; ++e) {
-    const int p = threadIdx.x + e * GB;
-    if (p < NPAR) out[p] = acc[e];
+  for (int i = 0; i < 4; ++i) {
+    const int o = ti + 16 * i;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[OW2 + o * NH + tj + 16 * j] = g2[i][j];
+    if (tj < 15)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) out[OW1 + o * NIN + tj + 15 * j] = g1[i][j];
   }
+  if (tk < 3)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) out[OW3 + (tk + 3 * i) * NH + tl] = g3[i][0];
+  if (tid < 2 * NH + NOUT)
+    out[tid < NH ? OB1 + tid : tid < 2 * NH ? OB2 + tid - NH : OB3 + tid - 2 * NH] = gb;
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, o);
-  __shared__ float lw[GB / 32];
-  if ((threadIdx.x & 31) == 0) lw[threadIdx.x >> 5] = lsum;
+  __shared__ float lw[GT / 32];
+  if ((tid & 31) == 0) lw[tid >> 5] = lsum;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     float l = 0.f;
-    for (int q = 0; q < GB / 32; ++q) l += lw[q];
+    for (int q = 0; q < GT / 32; ++q) l += lw[q];
     out[NPAR] = l * inv_n;
   }
 }
 
-// sums the per-block partials in block order (deterministic)
+// sums the per-block partials in block order (deterministic); the loads of 16
+// blocks are in flight together
 __global__ void reduce_partials(const float *__restrict__ partial, int nblocks,
                                 float *__restrict__ out) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= NPAR; p += gridDim.x * blockDim.x) {
     float s = 0.f;
+#pragma unroll 16
     for (int b = 0; b < nblocks; ++b) s += partial[(size_t)b * (NPAR + 1) + p];
     out[p] = s;
   }
@@ -597,8 +694,8 @@ extern "C" int cgfd_mlp_gradient(const void *weights_fp16, const float *x, const
   if (e == cudaSuccess) {
     int blocks = (n + GB - 1) / GB;
     if (blocks > B.nblocks) blocks = B.nblocks;
-    grad_kernel<<<blocks, GB, GRAD_SMEM>>>((const __half *)B.w, B.x, B.t, n, B.partial);
-    reduce_partials<<<(NPAR + 256) / 256, 256>>>(B.partial, blocks, B.out);
+    grad_kernel<<<blocks, GT, GRAD_SMEM>>>((const __half *)B.w, B.x, B.t, n, B.partial);
+    reduce_partials<<<(NPAR + 64) / 64, 64>>>(B.partial, blocks, B.out);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpy(grad, B.out, NPAR * sizeof(float), cudaMemcpyDeviceToHost);
