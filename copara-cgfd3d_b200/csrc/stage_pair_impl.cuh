@@ -615,6 +615,29 @@ __device__ __forceinline__ f2 mat_row(const float *mv, size_t plane, int r, f2 u
               fma2(lds2(mv + (r + 1) * plane), v, mul2(lds2(mv + r * plane), u)));
 }
 
+// stress rates of the velocity gradient (gx, gy: d/dx and d/dy of Vx, Vy, Vz;
+// gz: d/dzeta): lambda times its trace + 2 mu times its diagonal, mu times the
+// symmetric sums
+__device__ __forceinline__ void hooke(f2 lam, f2 mu, bool curved, f2 ztx, f2 zty, f2 ztz,
+                                      const f2 *gx, const f2 *gy, const f2 *gz, f2 *hw) {
+  f2 ga = gx[0], gb = gy[1], gxy = add2(gx[1], gy[0]), gxz = gx[2], gyz = gy[2];
+  const f2 gc = mul2(ztz, gz[2]), mu2 = add2(mu, mu);
+  if (curved) {
+    ga = fma2(ztx, gz[0], ga);
+    gb = fma2(zty, gz[1], gb);
+    gxy = fma2(ztx, gz[1], fma2(zty, gz[0], gxy));
+    gxz = fma2(ztx, gz[2], gxz);
+    gyz = fma2(zty, gz[2], gyz);
+  }
+  const f2 tr = mul2(lam, add2(add2(ga, gb), gc));
+  hw[0] = fma2(mu2, ga, tr);
+  hw[1] = fma2(mu2, gb, tr);
+  hw[2] = fma2(mu2, gc, tr);
+  hw[3] = mul2(mu, gxy);
+  hw[4] = mul2(mu, fma2(ztz, gz[0], gxz));
+  hw[5] = mul2(mu, fma2(ztz, gz[1], gyz));
+}
+
 template <typename T, int X, int Y, int Z, int KIND, bool LEAN>
 __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, const Plane &pl,
                                          uint32_t hp, const Pw2<T> &pw,
@@ -663,23 +686,14 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
                            fma2(S2(CGFD_MA1), W(q, 2), mul2(S2(CGFD_MA0), W(q, 3)))), sz(q));
     }
     const f2 rr = S2(RAW ? rh : 1.f);
-    const f2 mu = mul2(pw.C(1), rr), mu2 = add2(mu, mu);
-    const f2 lam = fma2(pw.C(0), rr, neg2(mu2));
+    const f2 mu = mul2(pw.C(1), rr);
+    const f2 lam = fma2(pw.C(0), rr, neg2(add2(mu, mu)));
     const f2 ztz = pl.zeta_z(pw);
-    // sigma_kk: lambda * (trace of the gradient) + 2 mu * its diagonal
-    f2 ga = DxVx, gb = DyVy, gxy = add2(DxVy, DyVx), gxz = DxVz, gyz = DyVz;
-    const f2 gc = mul2(ztz, DzV[2]);
-    if (pl.curved) {
-      const f2 ztx = pw.M(0), zty = pw.M(1);
-      ga = fma2(ztx, DzV[0], ga);
-      gb = fma2(zty, DzV[1], gb);
-      gxy = fma2(ztx, DzV[1], fma2(zty, DzV[0], gxy));
-      gxz = fma2(ztx, DzV[2], gxz);
-      gyz = fma2(zty, DzV[2], gyz);
-    }
-    const f2 tr = mul2(lam, add2(add2(ga, gb), gc));
-    const f2 hw[6] = {fma2(mu2, ga, tr), fma2(mu2, gb, tr), fma2(mu2, gc, tr), mul2(mu, gxy),
-                      mul2(mu, fma2(ztz, DzV[0], gxz)), mul2(mu, fma2(ztz, DzV[1], gyz))};
+    f2 ztx = S2(0.f), zty = S2(0.f);
+    if (pl.curved) { ztx = pw.M(0); zty = pw.M(1); }
+    const f2 gx3[3] = {DxVx, DxVy, DxVz}, gy3[3] = {DyVx, DyVy, DyVz};
+    f2 hw[6];
+    hooke(lam, mu, pl.curved, ztx, zty, ztz, gx3, gy3, DzV, hw);
 #pragma unroll
     for (int q = 0; q < 6; ++q)
       rk_store2<KIND>(a, out + (TXX + q) * fs + pl.c, tw + (TXX + q) * fs + pl.c, 3, pw.U0(q),
@@ -738,6 +752,37 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
   f2 ztx = S2(0.f), zty = S2(0.f);
   const f2 ztz = pl.zeta_z(pw);
   if (pl.curved) { ztx = pw.M(0); zty = pw.M(1); }
+  const f2 iBy = S2(e.iBy), iBz = S2(ix.iBz);
+  f2 hw[6];
+  if constexpr (sizeof(T) == 4) {
+    // The ADE is linear in the velocity derivatives, so the auxiliaries enter
+    // as a correction of the derivatives, (D - a) / B per direction, and
+    // Hooke's law is applied once to the corrected gradient: 45 instead of
+    // about 100 operations and 36 registers less than the three directional
+    // parts and their auxiliary terms of all six stresses.
+    f2 gx[3] = {DxVx, DxVy, DxVz}, gy[3] = {DyVx, DyVy, DyVz}, gz[3] = {DzVx, DzVy, DzVz};
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      if (mx) gx[q] = add2(gx[q], neg2(ax.ai[q]));
+      if (my) gy[q] = add2(gy[q], neg2(ay.ai[q]));
+      if (mz) gz[q] = add2(gz[q], neg2(az.ai[q]));
+      gx[q] = mul2(gx[q], e.iBx);
+      gy[q] = mul2(gy[q], iBy);
+      gz[q] = mul2(gz[q], iBz);
+    }
+    if (pl.top) {
+      // the xi (eta) part of the surface-matrix d/dzeta of V belongs to the x
+      // (y) auxiliaries (src/calculate.cu:4479-4491, 4527-4538)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        if (mx) gz[q] = add2(gz[q], neg2(mat_row(mv, g.plane, 3 * q, ax.ai[0], ax.ai[1], ax.ai[2])));
+        if (my)
+          gz[q] = add2(gz[q], neg2(mat_row(mv + 9 * g.plane, g.plane, 3 * q, ay.ai[0], ay.ai[1],
+                                           ay.ai[2])));
+      }
+    }
+    hooke(lambda, miu, pl.curved, ztx, zty, ztz, gx, gy, gz, hw);
+  } else {
   // components in the set order Txx Tyy Tzz Txy Txz Tyz (index q = comp - 3)
   f2 dxi[6], det[6], dzt[6];
   {
@@ -756,9 +801,7 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
     dzt[5] = mul2(fma2(zty, DzVz, mul2(ztz, DzVy)), miu);
   }
 
-  f2 hw[6];
   {
-    const f2 iBy = S2(e.iBy), iBz = S2(ix.iBz);
 #pragma unroll
     for (int q = 0; q < 6; ++q)
       hw[q] = fma2(dzt[q], iBz, fma2(det[q], iBy, mul2(dxi[q], e.iBx)));
@@ -817,6 +860,9 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
 #pragma unroll
       for (int q = 0; q < 6; ++q) hw[q] = fma2(neg2(t[q]), iBz, hw[q]);
     }
+  }
+  }
+  {
     // one direction at a time: the derivative auxiliaries' RHS
     // (-APD a + DB dV), then their RK update
     f2 ha[3];
