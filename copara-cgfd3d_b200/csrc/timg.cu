@@ -22,8 +22,8 @@ __device__ __forceinline__ float drp5(float m1, float c0, float p1, float p2, fl
   return (CGFD_DA_1 * m1 + CGFD_DA0 * c0 + CGFD_DA1 * p1 + CGFD_DA2 * p2 + CGFD_DA3 * p3) * r;
 }
 
-// one cell (i, j) of layer iz
-template <typename T>
+// one cell (i, j) of layer iz, velocity components Q0 .. Q1-1
+template <typename T, int Q0 = 0, int Q1 = 3>
 __device__ __forceinline__ void timg_cell(const StageArgs &a, int i, int j, int iz) {
   using E = Elem<T>;
   const Geom &g = a.g;
@@ -50,7 +50,7 @@ __device__ __forceinline__ void timg_cell(const StageArgs &a, int i, int j, int 
   T *out = static_cast<T *>(a.out), *tw = static_cast<T *>(a.tw);
 
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
+  for (int q = Q0; q < Q1; ++q) {
     const T *T1 = in + TC[q][0] * fs, *T2 = in + TC[q][1] * fs, *T3 = in + TC[q][2] * fs;
     // stored units to values (exact powers of two)
     const float s1 = a.sc[TC[q][0]], s2 = a.sc[TC[q][1]], s3 = a.sc[TC[q][2]];
@@ -139,6 +139,21 @@ __global__ void __launch_bounds__(128) timg_kernel(StageArgs a) {
                a.g.top - 2 + blockIdx.z);
 }
 
+// Small grids: a thread per component (blockIdx.z = component * 3 + layer).
+// There the kernel is one chain of loads and arithmetic per thread beside
+// stage kernels that are as short: the 118x95x61 hill 345 us a step with all three
+// components in a thread, 299 with one.  Each component loads the metric
+// again (1.6 times the loads in all), so grids that fill the GPU anyway keep
+// one thread per cell.
+template <typename T>
+__global__ void __launch_bounds__(128) timg_split_kernel(StageArgs a) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
+  const int iz = a.g.top - 2 + (int)(blockIdx.z % 3);
+  if (blockIdx.z < 3) timg_cell<T, 0, 1>(a, i, j, iz);
+  else if (blockIdx.z < 6) timg_cell<T, 1, 2>(a, i, j, iz);
+  else timg_cell<T, 2, 3>(a, i, j, iz);
+}
+
 // n models: blockIdx.z = model * 3 + layer; the grid covers the largest model
 template <typename T>
 __global__ void __launch_bounds__(128) timg_batch_kernel(const StageArgs *args) {
@@ -159,15 +174,26 @@ void launch_timg_batch(const StageArgs *args, int n, int max_ni, int max_nj, int
   else timg_batch_kernel<float><<<grid, block, 0, s>>>(args);
 }
 
-void launch_timg(const StageArgs &a, void *stream) {
+namespace {
+template <typename T>
+void timg_t(const StageArgs &a, cudaStream_t s) {
+  constexpr unsigned FULL = 148 * 8;  // blocks that keep every SM's warps busy
   dim3 block(32, 4, 1);
   dim3 grid((a.g.ni + 31) / 32, (a.g.nj + 3) / 4, 3);
-  if (a.elem == ELEM_F16)
-    timg_kernel<__half><<<grid, block, 0, (cudaStream_t)stream>>>(a);
-  else if (a.elem == ELEM_BF16)
-    timg_kernel<__nv_bfloat16><<<grid, block, 0, (cudaStream_t)stream>>>(a);
-  else
-    timg_kernel<float><<<grid, block, 0, (cudaStream_t)stream>>>(a);
+  if (grid.x * grid.y * 3 < FULL) {
+    grid.z = 9;
+    timg_split_kernel<T><<<grid, block, 0, s>>>(a);
+  } else {
+    timg_kernel<T><<<grid, block, 0, s>>>(a);
+  }
+}
+}  // namespace
+
+void launch_timg(const StageArgs &a, void *stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  if (a.elem == ELEM_F16) timg_t<__half>(a, s);
+  else if (a.elem == ELEM_BF16) timg_t<__nv_bfloat16>(a, s);
+  else timg_t<float>(a, s);
 }
 
 }  // namespace cgfd
