@@ -202,8 +202,8 @@ bool pair_set_work(void *plan, const WorkParams &wp);
 // per model: StageArgs::plain_interior (rebuilds the work lists on a change)
 bool pair_set_plain(void *plan, const char *plain);
 // test hook (cgfd_test_withhold_copy): every wait of the plan's kernels gives
-// up after wait_s, and with withhold >= 0 the velocity part's CTA 0 does not
-// issue the halo copy of entry `withhold` of its first item; withhold < 0
+// up after wait_s, and with withhold >= 0 the halo copy of entry `withhold` (at
+// most the last one) of the first velocity item is not issued; withhold < 0
 // restores the defaults
 bool pair_set_wait_test(void *plan, double wait_s, int withhold);
 WorkParams pair_get_work(const void *plan);

@@ -5,6 +5,7 @@
 #include "stage_pair_impl.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <new>
 #include <vector>
 
@@ -226,19 +227,22 @@ std::vector<int4> build_items(const std::vector<Geom> &gs, const std::vector<cha
       }
   }
   if (cols.empty()) return {};
-  // chunk length: about items_per_cta items per resident CTA, at
-  // least min_chunk planes; but where that leaves resident CTAs without an
-  // item, chunks down to MIN_LEN planes
-  constexpr int MIN_LEN = 4;
+  // chunk length: about items_per_cta items per resident CTA, at least
+  // min_chunk planes; but where that leaves resident CTAs without an item, as
+  // many planes as share the work out over all of them, down to one (the stage
+  // then takes a few planes' latency: 28x24x20 cells 103 us per step with
+  // chunks of at least 4 planes, 73 with 2, 60 with 1; 62x54x40 cells, where
+  // the work fills 1.4 planes per CTA, 132, 126 and 129, hence rounded up)
   const int parts = lean ? 2 : 1;
   const double fill = parts * planes / G;
   double len = std::max(fill / wp.items_per_cta, (double)wp.min_chunk);
-  if (fill < len) len = std::max(fill, (double)MIN_LEN);
+  if (fill < len) len = std::max(std::ceil(fill), 1.0);
+  const int min_len = (int)std::min(len, 4.0);
   std::vector<It> items;
   for (const Col &c : cols) {
     const int n = c.z1 - c.z0;
     int pieces = std::max(1, (int)(n / len + 0.5));
-    while (pieces > 1 && n / pieces < MIN_LEN) --pieces;
+    while (pieces > 1 && n / pieces < min_len) --pieces;
     if (zchunk && items.empty()) *zchunk = (n + pieces - 1) / pieces;
     for (int q = 0; q < pieces; ++q) {
       const int a0 = c.z0 + (int)((long)n * q / pieces);

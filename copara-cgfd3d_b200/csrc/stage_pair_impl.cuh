@@ -170,8 +170,9 @@ struct Work {
   const Maps *bmaps;   // [velocity, stress][model]
   int nmodels;
   // bound of every mbarrier wait, and the test hook of cgfd_test_withhold_copy:
-  // with withhold >= 0 the velocity part's CTA 0 does not issue the halo copy
-  // of entry `withhold` of its first item, so its wait for that plane expires
+  // with withhold >= 0 the halo copy of entry `withhold` (at most the last one)
+  // of a list's first velocity item is not issued, so the wait for that plane
+  // expires
   unsigned wait_us = WAIT_US;
   int withhold = -1;
 };
@@ -957,7 +958,8 @@ __device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const W
     fence_proxy_async();
     if (warp == 0) {
       mbar_expect_tx(&bars[s], S::HALO_B);
-      const bool withheld = PART == PART_VEL && withhold_item && wk.withhold == q;
+      const bool withheld =
+          PART == PART_VEL && withhold_item && wk.withhold >= 0 && min(wk.withhold, n) == q;
       if (!withheld) tma_load(slot, &M.halo, XO + i0 - HOFF, j0, p, C0, &bars[s]);
     } else if (warp == 1) {
       mbar_expect_tx(&bars[s], compute ? S::U_B : 0u);

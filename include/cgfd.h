@@ -324,9 +324,9 @@ int cgfd_set_work_shape(cgfd_solver *h, int items_per_cta, int min_chunk, double
  * reference's waits are cudaDeviceSynchronize calls that abort on error,
  * src/calculate.cu:17-41).  Every mbarrier wait of the default kernel gives
  * up after wait_limit_s (0 < wait_limit_s <= 60) instead of about 2 s, and
- * the velocity part's first CTA does not issue the halo tensor copy of entry
- * `withhold` of its first work item, so its wait for that plane runs out:
- * the CTA records the expiry, drains its own copies (bounded) and returns,
+ * the velocity part does not issue the halo tensor copy of entry `withhold`
+ * (at most the last one) of its first work item, so the wait for that plane
+ * runs out: the CTA records the expiry, drains its own copies (bounded) and returns,
  * and cgfd_sync reports CGFD_ERR_TIMEOUT.  The solver's state is then
  * invalid (destroy it); other solvers are unaffected.  withhold < 0 restores
  * normal operation.  Needs CGFD_KERNEL_FUSED; takes effect from the next
