@@ -76,6 +76,13 @@ struct Geom {
   // V's three, then one per velocity derivative in that direction, from
   // which the six stresses' auxiliaries follow linearly
   int ncaux;
+  // 16-bit storage: valid cells i in [kx0, kx1), j in [ky0, ky1) above the bottom
+  // layer add the directions' products with contracted sums in the velocity
+  // equations, the others round each product first.  Either order is as good,
+  // but a 16-bit run follows its roundings: with the tiles of 64 x 4 cells that
+  // lie inside the layers (as they were cut when those were the tiles) results
+  // stay what they were, to the last bit.
+  int kx0, kx1, ky0, ky1;
 };
 
 __host__ __device__ inline size_t gidx(const Geom &g, int ix, int iy, int iz) {

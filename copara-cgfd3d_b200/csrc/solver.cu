@@ -1023,6 +1023,31 @@ int cgfd_create(const cgfd_desc *d, cgfd_solver **out) {
   g.astride[1] = align_up((size_t)g.nzi * g.nya * g.px, 64);
   g.astride[2] = align_up((size_t)g.nza * g.nyi * g.px, 64);
   g.ncaux = (d->kernel == CGFD_KERNEL_FUSED) ? 6 : 9;
+  {
+    // tiles of 64 columns from -o, o = 32 where that takes no more tiles and
+    // leaves fewer columns in tiles that touch an x layer; of 4 rows from 0
+    auto inside = [&](int t, int o) {
+      return t * 64 - o >= g.nabs[0] && (t + 1) * 64 - o <= g.ni - g.nabs[1];
+    };
+    auto ntx = [&](int o) { return (g.ni + o + 63) / 64; };
+    auto edge = [&](int o) {
+      int n = 0;
+      for (int t = 0; t < ntx(o); ++t)
+        if (const int a = std::max(t * 64 - o, 0), b = std::min((t + 1) * 64 - o, g.ni);
+            a < g.nabs[0] || b > g.ni - g.nabs[1])
+          n += b - a;
+      return n;
+    };
+    const int o = ntx(32) == ntx(0) && edge(32) < edge(0) ? 32 : 0;
+    g.kx0 = g.kx1 = 0;
+    for (int t = 0; t < ntx(o); ++t)
+      if (inside(t, o)) {
+        if (g.kx1 == g.kx0) g.kx0 = t * 64 - o;
+        g.kx1 = (t + 1) * 64 - o;
+      }
+    g.ky0 = (g.nabs[2] + 3) / 4 * 4;
+    g.ky1 = (g.nj - g.nabs[3]) / 4 * 4;
+  }
   if ((d->kernel == CGFD_KERNEL_SCALAR && !fused_supported(g)) ||
       (d->kernel == CGFD_KERNEL_FUSED && !pair_supported(g))) {
     delete h;

@@ -407,6 +407,7 @@ struct Pair {
   int m;              // cells inside the grid (bit mask)
   int mx;             // cells inside an x layer (bit mask)
   bool ypml;          // the row is inside a y layer
+  bool kept;          // (lean, 16-bit) inside the range of Geom::kx0
   int xa0, xa1, ya;   // auxiliary x indices of the two cells, y index of the row
   f2 iBx, apdx, dbx, bbx;  // x profiles of the two cells (1/B, APD, DB, B)
   float iBy, apdy, dby, bby;
@@ -507,10 +508,10 @@ __device__ __forceinline__ void vel_pair(const StageArgs &a, const Pair &e, cons
           hw[q] = mul2(fma2(ztz, dz_raw(SZ[q]), add2(dx_raw(SX[q]), dy_raw(SY[q]))), ir);
       }
     } else {
-      // scaled derivatives (16-bit storage has a scale per component), and sums
-      // of the rounded products as in the general path with B = 1 (a plain add2 of
-      // products would be contracted)
-      const f2 one = S2(a.one);
+      // scaled derivatives (16-bit storage has a scale per component).  The order
+      // of rounding is kept (Geom::kx0): contracted sums inside that range, sums
+      // of the rounded products, as in the general path with B = 1, outside it
+      const f2 fb = e.kept ? irho : S2(a.one);
       f2 zs[3];
       if (pl.curved) {
         const f2 ztx = pw.M(0), zty = pw.M(1);
@@ -525,9 +526,14 @@ __device__ __forceinline__ void vel_pair(const StageArgs &a, const Pair &e, cons
         for (int q = 0; q < 3; ++q) zs[q] = mul2(ztz, dz(SZ[q]));
       }
 #pragma unroll
-      for (int q = 0; q < 3; ++q)
-        hw[q] = fma2(mul2(zs[q], irho), one,
-                     fma2(mul2(dx(SX[q]), irho), one, mul2(dy(SY[q]), irho)));
+      for (int q = 0; q < 3; ++q) {
+        f2 x = dx(SX[q]), z = zs[q];
+        if (!e.kept) {
+          x = mul2(x, irho);
+          z = mul2(z, irho);
+        }
+        hw[q] = fma2(z, fb, fma2(x, fb, mul2(dy(SY[q]), irho)));
+      }
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q)
@@ -616,6 +622,25 @@ __device__ __forceinline__ f2 mat_row(const float *mv, size_t plane, int r, f2 u
               fma2(lds2(mv + (r + 1) * plane), v, mul2(lds2(mv + r * plane), u)));
 }
 
+// the stress rates' parts by direction, in the set order Txx Tyy Tzz Txy Txz Tyz
+__device__ __forceinline__ void directional(f2 lam2mu, f2 lambda, f2 miu, f2 ztx, f2 zty, f2 ztz,
+                                            const f2 *gx, const f2 *gy, const f2 *gz, f2 *dxi,
+                                            f2 *det, f2 *dzt) {
+  const f2 tx2 = mul2(ztx, gz[0]), ty2 = mul2(zty, gz[1]), tz2 = mul2(ztz, gz[2]);
+  dxi[0] = mul2(lam2mu, gx[0]); det[0] = mul2(lambda, gy[1]);
+  dzt[0] = fma2(lambda, tz2, fma2(lambda, ty2, mul2(lam2mu, tx2)));
+  dxi[1] = mul2(lambda, gx[0]); det[1] = mul2(lam2mu, gy[1]);
+  dzt[1] = fma2(lambda, tz2, fma2(lam2mu, ty2, mul2(lambda, tx2)));
+  dxi[2] = mul2(lambda, gx[0]); det[2] = mul2(lambda, gy[1]);
+  dzt[2] = fma2(lam2mu, tz2, fma2(lambda, ty2, mul2(lambda, tx2)));
+  dxi[3] = mul2(gx[1], miu); det[3] = mul2(gy[0], miu);
+  dzt[3] = mul2(fma2(ztx, gz[1], mul2(zty, gz[0])), miu);
+  dxi[4] = mul2(gx[2], miu); det[4] = S2(0.f);
+  dzt[4] = mul2(fma2(ztx, gz[2], mul2(ztz, gz[0])), miu);
+  dxi[5] = S2(0.f); det[5] = mul2(gy[2], miu);
+  dzt[5] = mul2(fma2(zty, gz[2], mul2(ztz, gz[1])), miu);
+}
+
 // stress rates of the velocity gradient (gx, gy: d/dx and d/dy of Vx, Vy, Vz;
 // gz: d/dzeta): lambda times its trace + 2 mu times its diagonal, mu times the
 // symmetric sums
@@ -659,8 +684,10 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
   T *out = static_cast<T *>(a.out), *tw = static_cast<T *>(a.tw);
 
   if constexpr (LEAN) {
-    // FP32: raw derivatives, the moduli carry 1/h.  16-bit storage has a scale
-    // per component, which the derivatives carry with 1/h.
+    // FP32: raw derivatives, the moduli carry 1/h, Hooke's law in its trace form.
+    // 16-bit storage has a scale per component, which the derivatives carry with
+    // 1/h, and keeps its order of rounding: sums of the rounded products of the
+    // three directions, as in the general path with B = 1.
     constexpr bool RAW = sizeof(T) == 4;
     auto gx = [&](int s) { return RAW ? dx_raw(s) : dx(s); };
     auto gy = [&](int s) { return RAW ? dy_raw(s) : dy(s); };
@@ -687,14 +714,22 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
                            fma2(S2(CGFD_MA1), W(q, 2), mul2(S2(CGFD_MA0), W(q, 3)))), sz(q));
     }
     const f2 rr = S2(RAW ? rh : 1.f);
-    const f2 mu = mul2(pw.C(1), rr);
-    const f2 lam = fma2(pw.C(0), rr, neg2(add2(mu, mu)));
+    const f2 mu = RAW ? mul2(pw.C(1), rr) : pw.C(1);
+    const f2 lam = RAW ? fma2(pw.C(0), rr, neg2(add2(mu, mu))) : fma2(S2(-2.f), mu, pw.C(0));
     const f2 ztz = pl.zeta_z(pw);
     f2 ztx = S2(0.f), zty = S2(0.f);
     if (pl.curved) { ztx = pw.M(0); zty = pw.M(1); }
     const f2 gx3[3] = {DxVx, DxVy, DxVz}, gy3[3] = {DyVx, DyVy, DyVz};
     f2 hw[6];
-    hooke(lam, mu, pl.curved, ztx, zty, ztz, gx3, gy3, DzV, hw);
+    if constexpr (RAW) {
+      hooke(lam, mu, pl.curved, ztx, zty, ztz, gx3, gy3, DzV, hw);
+    } else {
+      f2 dxi[6], det[6], dzt[6];
+      directional(pw.C(0), lam, mu, ztx, zty, ztz, gx3, gy3, DzV, dxi, det, dzt);
+      const f2 one = S2(a.one);  // (add2 of products would be contracted)
+#pragma unroll
+      for (int q = 0; q < 6; ++q) hw[q] = fma2(dzt[q], one, fma2(det[q], one, dxi[q]));
+    }
 #pragma unroll
     for (int q = 0; q < 6; ++q)
       rk_store2<KIND>(a, out + (TXX + q) * fs + pl.c, tw + (TXX + q) * fs + pl.c, 3, pw.U0(q),
@@ -784,22 +819,10 @@ __device__ __forceinline__ void str_pair(const StageArgs &a, const Pair &e, cons
     }
     hooke(lambda, miu, pl.curved, ztx, zty, ztz, gx, gy, gz, hw);
   } else {
-  // components in the set order Txx Tyy Tzz Txy Txz Tyz (index q = comp - 3)
   f2 dxi[6], det[6], dzt[6];
   {
-    const f2 tx2 = mul2(ztx, DzVx), ty2 = mul2(zty, DzVy), tz2 = mul2(ztz, DzVz);
-    dxi[0] = mul2(lam2mu, DxVx); det[0] = mul2(lambda, DyVy);
-    dzt[0] = fma2(lambda, tz2, fma2(lambda, ty2, mul2(lam2mu, tx2)));
-    dxi[1] = mul2(lambda, DxVx); det[1] = mul2(lam2mu, DyVy);
-    dzt[1] = fma2(lambda, tz2, fma2(lam2mu, ty2, mul2(lambda, tx2)));
-    dxi[2] = mul2(lambda, DxVx); det[2] = mul2(lambda, DyVy);
-    dzt[2] = fma2(lam2mu, tz2, fma2(lambda, ty2, mul2(lambda, tx2)));
-    dxi[3] = mul2(DxVy, miu); det[3] = mul2(DyVx, miu);
-    dzt[3] = mul2(fma2(ztx, DzVy, mul2(zty, DzVx)), miu);
-    dxi[4] = mul2(DxVz, miu); det[4] = S2(0.f);
-    dzt[4] = mul2(fma2(ztx, DzVz, mul2(ztz, DzVx)), miu);
-    dxi[5] = S2(0.f); det[5] = mul2(DyVz, miu);
-    dzt[5] = mul2(fma2(zty, DzVz, mul2(ztz, DzVy)), miu);
+    const f2 gx[3] = {DxVx, DxVy, DxVz}, gy[3] = {DyVx, DyVy, DyVz}, gz[3] = {DzVx, DzVy, DzVz};
+    directional(lam2mu, lambda, miu, ztx, zty, ztz, gx, gy, gz, dxi, det, dzt);
   }
 
   {
@@ -980,7 +1003,7 @@ __device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const W
       if (!compute || warp == 0) return;
       const int d = warp - 1;  // direction
       const int c0 = (PART == PART_VEL) ? 0 : 3;
-      const int cxp = max(cx, 0);  // prefetch boxes start inside the arrays
+      const int cxp = max(cx, 0), cyp = max(cy, 0);  // prefetch boxes start inside the arrays
       const bool on = aux_on[d] &&
                       (d == 0   ? (i0 < g.nabs[0] || i0 + CX > g.ni - g.nabs[1])
                        : d == 1 ? (j0 < g.nabs[2] || j0 + TY > g.nj - g.nabs[3])
@@ -988,7 +1011,7 @@ __device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const W
       if (!on) return;
       const int bx = d == 0 ? ((i0 < g.nabs[0]) ? max(i0, 0) : i0 - (g.ni - g.nabs[1]) + g.xaoff)
                             : cxp;
-      const int by = d == 1 ? ((j0 < g.nabs[2]) ? max(j0, 0) : j0 - (g.nj - g.nabs[3]) + g.nabs[2]) : cy;
+      const int by = d == 1 ? ((j0 < g.nabs[2]) ? max(j0, 0) : j0 - (g.nj - g.nabs[3]) + g.nabs[2]) : cyp;
       const int bz = d == 2 ? ((p - LFD < g.nabs[4]) ? p - LFD
                                                      : p - LFD - (g.nk - g.nabs[5]) + g.nabs[4])
                             : p;
@@ -1015,6 +1038,7 @@ __device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const W
   e.ix = e.i + XO;
   e.iy = e.j + LFD;
   e.m = 3;
+  e.kept = e.i >= g.kx0 && e.i < g.kx1 && e.j >= g.ky0 && e.j < g.ky1;
   if constexpr (!LEAN) {
     const bool rowok = e.j >= 0 && e.j < g.nj;  // (tile origins may lie left of the grid)
     e.m = (rowok && e.i >= 0 && e.i < g.ni ? 1 : 0) |
