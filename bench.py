@@ -166,10 +166,11 @@ def run_batch(args, dist, rank, world, local):
                      "frac": achieved / peak, "traffic": None,
                      "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)",
                      "algorithmic_bytes_per_step": bps,
-                     "launch": "whole batched step (4 stages: velocity + stress pair_kernel, "
-                               "timg, sources; receiver record)"},
+                     "launch": "whole batched step (4 stages: pair_kernel over the general items "
+                               "(velocity, stress) and the lean ones, timg, sources; "
+                               "receiver record)"},
         "clocks": clk.summary(),
-        "gpu_launches": K * (4 * (3 + (1 if n_src else 0)) + 1),
+        "gpu_launches": K * (4 * (4 + (1 if n_src else 0)) + 1),
         "nonfinite": nbad,
     }
     print(json.dumps(line))
@@ -631,7 +632,8 @@ def main():
                      "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)",
                      "algorithmic_bytes_per_step": bps, "stage_kernel_ms": stage_ms},
         "clocks": clk.summary(),
-        "gpu_launches": K * (4 * (1 if args.kernel == "simple" else 3) + 4 * n_src + 1 +
+        # per stage: general velocity and stress, lean items, traction image
+        "gpu_launches": K * (4 * {"simple": 1, "scalar": 3}.get(args.kernel, 4) + 4 * n_src + 1 +
                              (2 if args.mlp else 0)),
         "nonfinite": nbad,
     }
