@@ -88,13 +88,14 @@ const Entry &entry(int elem, int kind, int list) {
   return e[elem][kind][list];
 }
 
-void set_all_attrs() {
-  static bool done = false;
-  if (done) return;
-  for (int elem = 0; elem < 3; ++elem)
-    for (int kind = 0; kind < 3; ++kind)
-      for (int list = 0; list < NLIST; ++list) entry(elem, kind, list).attrs();
-  done = true;
+// kernel attributes of one storage type (each call loads its kernels, so a
+// process pays for the types it uses only)
+void set_attrs_of(int elem) {
+  static bool done[3];
+  if (done[elem]) return;
+  for (int kind = 0; kind < 3; ++kind)
+    for (int list = 0; list < NLIST; ++list) entry(elem, kind, list).attrs();
+  done[elem] = true;
 }
 
 // tensor maps of one model's buffers
@@ -334,7 +335,7 @@ bool upload_items(Plan *pl, const std::vector<int4> (&hv)[2],
 
 void *pair_create_plan(const Geom &g, int elem, void *const sets[4], const float *media,
                        const float *metric, float *const aux[3]) {
-  set_all_attrs();
+  set_attrs_of(elem);
   Plan *pl = new (std::nothrow) Plan();
   if (!pl) return nullptr;
   pl->elem = elem;
@@ -425,7 +426,7 @@ void launch_stage_pair(const void *plan, const StageArgs &a, int in_set, int *er
 
 void *pair_create_batch_plan(int n, const Geom *gs, void *const *sets, const float *const *media,
                              const float *const *metric, float *const *aux, int elem) {
-  set_all_attrs();
+  set_attrs_of(elem);
   Plan *pl = new (std::nothrow) Plan();
   if (!pl) return nullptr;
   pl->elem = elem;
