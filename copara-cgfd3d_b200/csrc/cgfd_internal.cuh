@@ -79,9 +79,9 @@ struct Geom {
   // 16-bit storage: valid cells i in [kx0, kx1), j in [ky0, ky1) above the bottom
   // layer add the directions' products with contracted sums in the velocity
   // equations, the others round each product first.  Either order is as good,
-  // but a 16-bit run follows its roundings: with the tiles of 64 x 4 cells that
-  // lie inside the layers (as they were cut when those were the tiles) results
-  // stay what they were, to the last bit.
+  // but a 16-bit run follows its roundings: the range is that of the tiles of
+  // 64 x 4 cells inside the layers that brought the order in, and every kernel
+  // and item list keeps it, so results do not depend on how the grid is cut.
   int kx0, kx1, ky0, ky1;
 };
 

@@ -407,7 +407,7 @@ struct Pair {
   int m;              // cells inside the grid (bit mask)
   int mx;             // cells inside an x layer (bit mask)
   bool ypml;          // the row is inside a y layer
-  bool kept;          // (lean, 16-bit) inside the range of Geom::kx0
+  bool kept;          // (16-bit) inside the range of Geom::kx0
   int xa0, xa1, ya;   // auxiliary x indices of the two cells, y index of the row
   f2 iBx, apdx, dbx, bbx;  // x profiles of the two cells (1/B, APD, DB, B)
   float iBy, apdy, dby, bby;
@@ -553,27 +553,37 @@ __device__ __forceinline__ void vel_pair(const StageArgs &a, const Pair &e, cons
   const f2 ztz = pl.zeta_z(pw);
   if (pl.curved) { ztx = pw.M(0); zty = pw.M(1); }
   f2 dxi[3], det[3], dzt[3];
-  dxi[0] = mul2(dx(0), irho);  // DxTxx
-  dxi[1] = mul2(dx(3), irho);  // DxTxy
-  dxi[2] = mul2(dx(4), irho);  // DxTxz
+  dxi[0] = dx(0);              // DxTxx
+  dxi[1] = dx(3);              // DxTxy
+  dxi[2] = dx(4);              // DxTxz
   det[0] = mul2(dy(3), irho);  // DyTxy
   det[1] = mul2(dy(1), irho);  // DyTyy
   det[2] = mul2(dy(5), irho);  // DyTyz
   const f2 DzTzz = dz(2), DzTxz = dz(4), DzTyz = dz(5);
   if (pl.curved) {
     const f2 DzTxx = dz(0), DzTyy = dz(1), DzTxy = dz(3);
-    dzt[0] = mul2(fma2(ztz, DzTxz, fma2(zty, DzTxy, mul2(ztx, DzTxx))), irho);
-    dzt[1] = mul2(fma2(ztz, DzTyz, fma2(zty, DzTyy, mul2(ztx, DzTxy))), irho);
-    dzt[2] = mul2(fma2(ztz, DzTzz, fma2(zty, DzTyz, mul2(ztx, DzTxz))), irho);
+    dzt[0] = fma2(ztz, DzTxz, fma2(zty, DzTxy, mul2(ztx, DzTxx)));
+    dzt[1] = fma2(ztz, DzTyz, fma2(zty, DzTyy, mul2(ztx, DzTxy)));
+    dzt[2] = fma2(ztz, DzTzz, fma2(zty, DzTyz, mul2(ztx, DzTxz)));
   } else {
-    dzt[0] = mul2(mul2(ztz, DzTxz), irho);
-    dzt[1] = mul2(mul2(ztz, DzTyz), irho);
-    dzt[2] = mul2(mul2(ztz, DzTzz), irho);
+    dzt[0] = mul2(ztz, DzTxz);
+    dzt[1] = mul2(ztz, DzTyz);
+    dzt[2] = mul2(ztz, DzTzz);
   }
   const f2 iBy = S2(e.iBy), iBz = S2(ix.iBz);
   f2 hw[3], hax[3], hay[3], haz[3];
+  // 16-bit storage: the order of rounding of Geom::kx0 (such a pair has no
+  // auxiliaries and B = 1); rows of the range that fill no tile, and models too
+  // shallow for lean items, come through here
+  const bool kept = sizeof(T) != 4 && e.kept && !pl.zpml;
 #pragma unroll
-  for (int q = 0; q < 3; ++q) hw[q] = fma2(dzt[q], iBz, fma2(det[q], iBy, mul2(dxi[q], e.iBx)));
+  for (int q = 0; q < 3; ++q) {
+    const f2 c = fma2(dzt[q], irho, fma2(dxi[q], irho, det[q]));
+    dxi[q] = mul2(dxi[q], irho);
+    dzt[q] = mul2(dzt[q], irho);
+    const f2 r = fma2(dzt[q], iBz, fma2(det[q], iBy, mul2(dxi[q], e.iBx)));
+    hw[q] = kept ? c : r;
+  }
   if (mx) {
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -1038,7 +1048,7 @@ __device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const W
   e.ix = e.i + XO;
   e.iy = e.j + LFD;
   e.m = 3;
-  e.kept = e.i >= g.kx0 && e.i < g.kx1 && e.j >= g.ky0 && e.j < g.ky1;
+  e.kept = A.plain_interior && e.i >= g.kx0 && e.i < g.kx1 && e.j >= g.ky0 && e.j < g.ky1;
   if constexpr (!LEAN) {
     const bool rowok = e.j >= 0 && e.j < g.nj;  // (tile origins may lie left of the grid)
     e.m = (rowok && e.i >= 0 && e.i < g.ni ? 1 : 0) |
