@@ -494,7 +494,10 @@ struct DevGuard {
   }
 };
 
+// (the error reported is taken off the runtime, so that no later call reports
+// it once more)
 int cuda_fail(cgfd_solver *h, cudaError_t e, const char *what) {
+  cudaGetLastError();
   char buf[512];
   std::snprintf(buf, sizeof(buf), "%s: %s (%d)", what, cudaGetErrorString(e), (int)e);
   if (h) h->err = buf; else g_last_create_error = buf;
@@ -503,6 +506,12 @@ int cuda_fail(cgfd_solver *h, cudaError_t e, const char *what) {
 int arg_fail(cgfd_solver *h, const char *what) {
   if (h) h->err = what; else g_last_create_error = what;
   return CGFD_ERR_ARG;
+}
+
+// why a work list could not be rebuilt (the plan keeps the earlier one)
+cudaError_t list_error() {
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? cudaErrorUnknown : e;
 }
 
 #define CK(h, call)                                         \
@@ -1708,7 +1717,7 @@ int cgfd_prepare(cgfd_solver *h) {
   }
   if (h->d.kernel == CGFD_KERNEL_FUSED) {
     const char plain = h->plain_interior;
-    if (!pair_set_plain(h->plan, &plain)) return cuda_fail(h, cudaErrorUnknown, "work list");
+    if (!pair_set_plain(h->plan, &plain)) return cuda_fail(h, list_error(), "work list");
   }
   h->prepared = true;
   int st = build_graphs(h);
@@ -2056,7 +2065,10 @@ int cgfd_autotune(cgfd_solver *h, int steps, float *best_ms) {
   float best = 1e30f;
   WorkParams bestp = pair_get_work(h->plan);
   for (const WorkParams &wp : tuning_candidates(bestp)) {
-    if (!pair_set_work(h->plan, wp)) continue;
+    if (!pair_set_work(h->plan, wp)) {
+      list_error();
+      continue;
+    }
     h->graphs_ok = false;
     st = build_graphs(h);
     if (st) break;
@@ -2069,7 +2081,10 @@ int cgfd_autotune(cgfd_solver *h, int steps, float *best_ms) {
   }
   int st2 = snapshot_restore(h, sn);
   if (!st) st = st2;
-  if (!pair_set_work(h->plan, bestp) && !st) st = cuda_fail(h, cudaErrorUnknown, "work list");
+  if (!pair_set_work(h->plan, bestp)) {
+    const cudaError_t e = list_error();
+    if (!st) st = cuda_fail(h, e, "work list");
+  }
   h->graphs_ok = false;
   if (!st) st = build_graphs(h);
   if (best_ms) *best_ms = best / steps;
@@ -2104,7 +2119,10 @@ int cgfd_set_work_shape(cgfd_solver *h, int items_per_cta, int min_chunk, double
   w.items_per_cta = items_per_cta;
   w.min_chunk = min_chunk;
   w.pml_weight = pml_weight;
-  if (!pair_set_work(h->plan, w)) return arg_fail(h, "work list rejected for this model");
+  if (!pair_set_work(h->plan, w)) {
+    // (any shape in the range above has a list)
+    return cuda_fail(h, list_error(), "work list");
+  }
   h->graphs_ok = false;  // the step graphs hold the launch configuration
   return build_graphs(h);
   CGFD_ABI_END(h)
@@ -2172,8 +2190,10 @@ static int batch_fail(cgfd_batch *b, int code, const std::string &msg) {
 #define BCK(b, call)                                                                  \
   do {                                                                                \
     cudaError_t e_ = (call);                                                          \
-    if (e_ != cudaSuccess)                                                            \
+    if (e_ != cudaSuccess) {                                                          \
+      cudaGetLastError();                                                             \
       return batch_fail((b), CGFD_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+    }                                                                                 \
   } while (0)
 
 static void batch_free(cgfd_batch *b) {
@@ -2277,7 +2297,8 @@ static int batch_build(cgfd_batch *b) {
   std::vector<char> plain(n);
   for (int i = 0; i < n; ++i) plain[i] = b->m[i]->plain_interior;
   if (!pair_set_plain(b->plan, plain.data()))
-    return batch_fail(b, CGFD_ERR_CUDA, "batch work list");
+    return batch_fail(b, CGFD_ERR_CUDA,
+                      std::string("batch work list: ") + cudaGetErrorString(list_error()));
   if (!pair_batch_set_args(b->plan, args.data()))
     return batch_fail(b, CGFD_ERR_CUDA, "batch stage arguments");
   if (!b->d_src) BCK(b, cudaMalloc(&b->d_src, src.size() * sizeof(SourceArgs)));
@@ -2491,7 +2512,10 @@ int cgfd_batch_autotune(cgfd_batch *b, int steps, float *best_ms) {
   float best = 1e30f;
   WorkParams bestp = pair_get_work(b->plan);
   for (const WorkParams &wp : tuning_candidates(bestp)) {
-    if (!pair_set_work(b->plan, wp)) continue;
+    if (!pair_set_work(b->plan, wp)) {
+      list_error();
+      continue;
+    }
     b->ready = false;
     st = batch_build(b);
     if (st) break;
@@ -2525,7 +2549,10 @@ int cgfd_batch_autotune(cgfd_batch *b, int steps, float *best_ms) {
     if (!st) st = st2;
   }
   b->member_launch = members_best;
-  if (!pair_set_work(b->plan, bestp) && !st) st = batch_fail(b, CGFD_ERR_CUDA, "work list");
+  if (!pair_set_work(b->plan, bestp)) {
+    const cudaError_t e = list_error();
+    if (!st) st = batch_fail(b, CGFD_ERR_CUDA, std::string("work list: ") + cudaGetErrorString(e));
+  }
   b->ready = false;
   if (!st) st = batch_build(b);
   if (best_ms) *best_ms = best / steps;

@@ -298,35 +298,55 @@ std::vector<int4> build_items(const std::vector<Geom> &gs, const std::vector<cha
   return hv;
 }
 
-// uploads the two work lists into the plan (replacing earlier ones)
+// uploads the two work lists into the plan; the earlier ones are replaced, and
+// freed, only when the new ones are complete
 bool upload_items(Plan *pl, const std::vector<int4> (&hv)[2],
                   const int (&G)[NLIST]) {
   Work &wk = pl->wk;
   if (hv[0].empty() && hv[1].empty()) return false;
+  int4 *d[2] = {nullptr, nullptr};
+  bool ok = true;
+  for (int l = 0; l < 2; ++l)
+    if (ok && !hv[l].empty())
+      ok = cudaMalloc(&d[l], hv[l].size() * sizeof(int4)) == cudaSuccess &&
+           cudaMemcpy(d[l], hv[l].data(), hv[l].size() * sizeof(int4), cudaMemcpyHostToDevice) ==
+               cudaSuccess;
+  if (ok && !wk.counter) {
+    int *c = nullptr;
+    ok = cudaMalloc(&c, 2 * NLIST * sizeof(int)) == cudaSuccess &&
+         cudaMemset(c, 0, 2 * NLIST * sizeof(int)) == cudaSuccess;
+    if (ok) wk.counter = c;
+    else cudaFree(c);
+  }
+  if (!ok) {
+    for (int4 *p : d) cudaFree(p);
+    return false;
+  }
   for (int l = 0; l < 2; ++l) {
     cudaFree((void *)wk.items[l]);
-    wk.items[l] = nullptr;
+    wk.items[l] = d[l];
     wk.nitems[l] = (int)hv[l].size();
-    if (hv[l].empty()) continue;
-    int4 *d_items = nullptr;
-    if (cudaMalloc(&d_items, hv[l].size() * sizeof(int4)) != cudaSuccess ||
-        cudaMemcpy(d_items, hv[l].data(), hv[l].size() * sizeof(int4), cudaMemcpyHostToDevice) !=
-            cudaSuccess) {
-      cudaFree(d_items);
-      wk.nitems[l] = 0;
-      return false;
-    }
-    wk.items[l] = d_items;
   }
   for (int q = 0; q < NLIST; ++q) {
     const int n = wk.nitems[q == LEAN_BOTH];
     pl->grid[q] = n < G[q] ? n : G[q];
   }
-  if (!wk.counter) {
-    if (cudaMalloc(&wk.counter, 2 * NLIST * sizeof(int)) != cudaSuccess ||
-        cudaMemset(wk.counter, 0, 2 * NLIST * sizeof(int)) != cudaSuccess)
-      return false;
-  }
+  return true;
+}
+
+// builds the work lists of a shape and of the models' `plain` flags; on failure
+// the plan keeps its lists, shape and flags
+bool rebuild(Plan *pl, const WorkParams &wp, const std::vector<char> &plain) {
+  std::vector<int4> hv[2];
+  int G[NLIST], zchunk = pl->zchunk;
+  for (int q = 0; q < NLIST; ++q) G[q] = entry(pl->elem, 1, q).resident[pl->nmodels > 0]();
+  for (int l = 0; l < 2; ++l)
+    hv[l] = build_items(pl->geoms, plain, l != 0,
+                        l ? G[LEAN_BOTH] : std::min(G[GEN_VEL], G[GEN_STR]), wp, &zchunk);
+  if (!upload_items(pl, hv, G)) return false;
+  pl->zchunk = zchunk;
+  pl->params = wp;
+  pl->plain = plain;
   return true;
 }
 
@@ -356,23 +376,13 @@ WorkParams pair_get_work(const void *plan) {
 
 bool pair_set_work(void *plan, const WorkParams &wp) {
   Plan *pl = reinterpret_cast<Plan *>(plan);
-  std::vector<int4> hv[2];
-  int G[NLIST];
-  for (int q = 0; q < NLIST; ++q) G[q] = entry(pl->elem, 1, q).resident[pl->nmodels > 0]();
-  for (int l = 0; l < 2; ++l)
-    hv[l] = build_items(pl->geoms, pl->plain, l != 0,
-                        l ? G[LEAN_BOTH] : std::min(G[GEN_VEL], G[GEN_STR]), wp, &pl->zchunk);
-  if (!upload_items(pl, hv, G)) return false;
-  pl->params = wp;
-  return true;
+  return rebuild(pl, wp, std::vector<char>(pl->plain));
 }
 
 bool pair_set_plain(void *plan, const char *plain) {
   Plan *pl = reinterpret_cast<Plan *>(plan);
   const std::vector<char> v(plain, plain + pl->geoms.size());
-  if (v == pl->plain) return true;
-  pl->plain = v;
-  return pair_set_work(plan, pl->params);
+  return v == pl->plain || rebuild(pl, pl->params, v);
 }
 
 bool pair_set_wait_test(void *plan, double wait_s, int withhold) {

@@ -1254,7 +1254,7 @@ struct Plan {
   std::vector<char> plain;     // per model: StageArgs::plain_interior
   Work wk;
   int elem;                    // storage element type of the field sets
-  int zchunk;                  // planes of the (first model's) interior z-chunks
+  int zchunk = 0;              // planes of the (first model's) interior z-chunks
   int grid[NLIST];             // CTAs per launch (0: no items)
   WorkParams params;
   int nmodels = 0;             // 0: single-model plan; else a batch of nmodels
