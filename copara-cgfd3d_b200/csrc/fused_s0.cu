@@ -10,7 +10,7 @@ void launch_s0(const Plan &pl, const StageMaps &m, const StageArgs &a, int *err,
   launch_dirs<PART_STR, 0>(pl, m, a, err, s);
 }
 
-void attrs_s0() { set_attrs<PART_STR, 0>(); }
+cudaError_t attrs_s0() { return set_attrs<PART_STR, 0>(); }
 
 }  // namespace fused
 }  // namespace cgfd

@@ -10,7 +10,7 @@ void launch_s1(const Plan &pl, const StageMaps &m, const StageArgs &a, int *err,
   launch_dirs<PART_STR, 1>(pl, m, a, err, s);
 }
 
-void attrs_s1() { set_attrs<PART_STR, 1>(); }
+cudaError_t attrs_s1() { return set_attrs<PART_STR, 1>(); }
 
 int resident_str() { return resident_ctas<PART_STR>(); }
 

@@ -10,7 +10,7 @@ void launch_s2(const Plan &pl, const StageMaps &m, const StageArgs &a, int *err,
   launch_dirs<PART_STR, 2>(pl, m, a, err, s);
 }
 
-void attrs_s2() { set_attrs<PART_STR, 2>(); }
+cudaError_t attrs_s2() { return set_attrs<PART_STR, 2>(); }
 
 }  // namespace fused
 }  // namespace cgfd

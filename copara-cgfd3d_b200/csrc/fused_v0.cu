@@ -10,7 +10,7 @@ void launch_v0(const Plan &pl, const StageMaps &m, const StageArgs &a, int *err,
   launch_dirs<PART_VEL, 0>(pl, m, a, err, s);
 }
 
-void attrs_v0() { set_attrs<PART_VEL, 0>(); }
+cudaError_t attrs_v0() { return set_attrs<PART_VEL, 0>(); }
 
 }  // namespace fused
 }  // namespace cgfd

@@ -10,7 +10,7 @@ void launch_v1(const Plan &pl, const StageMaps &m, const StageArgs &a, int *err,
   launch_dirs<PART_VEL, 1>(pl, m, a, err, s);
 }
 
-void attrs_v1() { set_attrs<PART_VEL, 1>(); }
+cudaError_t attrs_v1() { return set_attrs<PART_VEL, 1>(); }
 
 int resident_vel() { return resident_ctas<PART_VEL>(); }
 

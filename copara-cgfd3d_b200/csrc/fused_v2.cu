@@ -10,7 +10,7 @@ void launch_v2(const Plan &pl, const StageMaps &m, const StageArgs &a, int *err,
   launch_dirs<PART_VEL, 2>(pl, m, a, err, s);
 }
 
-void attrs_v2() { set_attrs<PART_VEL, 2>(); }
+cudaError_t attrs_v2() { return set_attrs<PART_VEL, 2>(); }
 
 }  // namespace fused
 }  // namespace cgfd

@@ -1121,9 +1121,11 @@ int cgfd_create(const cgfd_desc *d, cgfd_solver **out) {
                   ? pair_create_plan(g, h->elem, h->set, h->media, h->metric, h->aux)
                   : fused_create_plan(g, fsets, h->media, h->metric);
     if (!h->plan) {
+      const cudaError_t e2 = cudaGetLastError();
       free_all(h);
       delete h;
-      g_last_create_error = "cuTensorMapEncodeTiled failed";
+      if (e2 != cudaSuccess) return cuda_fail(nullptr, e2, "stage kernels");
+      g_last_create_error = "stage kernels: no tensor maps, or no room for them on the device";
       return CGFD_ERR_CUDA;
     }
   }

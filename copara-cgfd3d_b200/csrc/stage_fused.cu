@@ -2,6 +2,7 @@
 // tensor maps, launch plan (persistent grid, z-chunk length) and dispatch.
 // The kernels themselves are in stage_fused_impl.cuh, instantiated by
 // fused_{v,s}{0,1,2}.cu.
+#include "once_per_device.h"
 #include "stage_fused_impl.cuh"
 
 #include <new>
@@ -59,12 +60,13 @@ bool fused_supported(const Geom &g) {
 
 void *fused_create_plan(const Geom &g, float *const sets[4], const float *media,
                         const float *metric) {
-  static bool attrs = false;
-  if (!attrs) {
-    attrs_v0(); attrs_v1(); attrs_v2();
-    attrs_s0(); attrs_s1(); attrs_s2();
-    attrs = true;
-  }
+  static OncePerDevice once;
+  const bool set = once.run(0, [] {
+    for (auto attrs : {attrs_v0, attrs_v1, attrs_v2, attrs_s0, attrs_s1, attrs_s2})
+      if (const cudaError_t e = attrs()) return e;
+    return cudaSuccess;
+  });
+  if (!set) return nullptr;
   Plan *pl = new (std::nothrow) Plan();
   if (!pl) return nullptr;
   bool ok = true;
@@ -83,8 +85,11 @@ void *fused_create_plan(const Geom &g, float *const sets[4], const float *media,
   }
   pl->ntx = (g.ni + TX - 1) / TX;
   pl->ntiles = pl->ntx * ((g.nj + TY - 1) / TY);
-  const int G = resident_vel() < resident_str() ? resident_vel()
-                                                                     : resident_str();
+  const int G = resident_vel() < resident_str() ? resident_vel() : resident_str();
+  if (G < 1) {
+    delete pl;
+    return nullptr;
+  }
   // z-chunk length: minimise (rounds of work over the resident CTAs) x
   // (chunk length + start-up planes)
   double best = 1e30;

@@ -624,9 +624,12 @@ void launch_dirs(const Plan &pl, const StageMaps &m, const StageArgs &a, int *er
 }
 
 template <int PART, int KIND>
-void set_attrs() {
-  auto set = [](const void *f) {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Slot<PART>::SMEM);
+cudaError_t set_attrs() {
+  cudaError_t e = cudaSuccess;
+  auto set = [&](const void *f) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)Slot<PART>::SMEM);
   };
   set((const void *)stage_part_kernel<PART, -1, -1, -1, KIND>);
   set((const void *)stage_part_kernel<PART, -1, -1, 1, KIND>);
@@ -636,6 +639,7 @@ void set_attrs() {
   set((const void *)stage_part_kernel<PART, 1, -1, 1, KIND>);
   set((const void *)stage_part_kernel<PART, 1, 1, -1, KIND>);
   set((const void *)stage_part_kernel<PART, 1, 1, 1, KIND>);
+  return e;
 }
 
 template <int PART>
@@ -645,8 +649,6 @@ int resident_ctas() {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &per, stage_part_kernel<PART, 1, 1, 1, 1>, TT, Slot<PART>::SMEM);
-  if (per < 1) per = 1;
-  if (sms < 1) sms = 1;
   return per * sms;
 }
 
@@ -654,7 +656,7 @@ int resident_ctas() {
 #define CGFD_FUSED_DECL(P, K)                                                        \
   void launch_##P##K(const Plan &pl, const StageMaps &m, const StageArgs &a, int *err, \
                      cudaStream_t s);                                                \
-  void attrs_##P##K();
+  cudaError_t attrs_##P##K();
 CGFD_FUSED_DECL(v, 0)
 CGFD_FUSED_DECL(v, 1)
 CGFD_FUSED_DECL(v, 2)

@@ -2,6 +2,7 @@
 // tensor maps, launch plan (persistent grid, z-chunk length) and dispatch.
 // The kernels themselves are in stage_pair_impl.cuh, instantiated by
 // pair_*.cu.
+#include "once_per_device.h"
 #include "stage_pair_impl.cuh"
 
 #include <algorithm>
@@ -88,14 +89,17 @@ const Entry &entry(int elem, int kind, int list) {
   return e[elem][kind][list];
 }
 
-// kernel attributes of one storage type (each call loads its kernels, so a
-// process pays for the types it uses only)
-void set_attrs_of(int elem) {
-  static bool done[3];
-  if (done[elem]) return;
-  for (int kind = 0; kind < 3; ++kind)
-    for (int list = 0; list < NLIST; ++list) entry(elem, kind, list).attrs();
-  done[elem] = true;
+// kernel attributes of one storage type on the current device (each call loads
+// its kernels, so a process pays for the types and devices it uses only)
+bool set_attrs_of(int elem) {
+  static OncePerDevice once;
+  return once.run(elem, [&] {
+    cudaError_t e = cudaSuccess;
+    for (int kind = 0; kind < 3; ++kind)
+      for (int list = 0; list < NLIST && e == cudaSuccess; ++list)
+        e = entry(elem, kind, list).attrs();
+    return e;
+  });
 }
 
 // tensor maps of one model's buffers
@@ -339,7 +343,10 @@ bool upload_items(Plan *pl, const std::vector<int4> (&hv)[2],
 bool rebuild(Plan *pl, const WorkParams &wp, const std::vector<char> &plain) {
   std::vector<int4> hv[2];
   int G[NLIST], zchunk = pl->zchunk;
-  for (int q = 0; q < NLIST; ++q) G[q] = entry(pl->elem, 1, q).resident[pl->nmodels > 0]();
+  for (int q = 0; q < NLIST; ++q) {
+    G[q] = entry(pl->elem, 1, q).resident[pl->nmodels > 0]();
+    if (G[q] < 1) return false;
+  }
   for (int l = 0; l < 2; ++l)
     hv[l] = build_items(pl->geoms, plain, l != 0,
                         l ? G[LEAN_BOTH] : std::min(G[GEN_VEL], G[GEN_STR]), wp, &zchunk);
@@ -355,7 +362,7 @@ bool rebuild(Plan *pl, const WorkParams &wp, const std::vector<char> &plain) {
 
 void *pair_create_plan(const Geom &g, int elem, void *const sets[4], const float *media,
                        const float *metric, float *const aux[3]) {
-  set_attrs_of(elem);
+  if (!set_attrs_of(elem)) return nullptr;
   Plan *pl = new (std::nothrow) Plan();
   if (!pl) return nullptr;
   pl->elem = elem;
@@ -436,7 +443,7 @@ void launch_stage_pair(const void *plan, const StageArgs &a, int in_set, int *er
 
 void *pair_create_batch_plan(int n, const Geom *gs, void *const *sets, const float *const *media,
                              const float *const *metric, float *const *aux, int elem) {
-  set_attrs_of(elem);
+  if (!set_attrs_of(elem)) return nullptr;
   Plan *pl = new (std::nothrow) Plan();
   if (!pl) return nullptr;
   pl->elem = elem;

@@ -1289,10 +1289,12 @@ void launch_dirs(const Plan &pl, const Maps *m, const StageArgs &a, const Work &
 }
 
 template <typename T, int KIND, bool B, int LIST>
-void set_attrs() {
-  auto set = [](const void *f) {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Ring<T, LIST>::SMEM);
+cudaError_t set_attrs() {
+  cudaError_t e = cudaSuccess;
+  auto set = [&](const void *f) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)Ring<T, LIST>::SMEM);
   };
   set((const void *)pair_kernel<T, -1, -1, -1, KIND, B, LIST>);
   set((const void *)pair_kernel<T, -1, -1, 1, KIND, B, LIST>);
@@ -1302,8 +1304,10 @@ void set_attrs() {
   set((const void *)pair_kernel<T, 1, -1, 1, KIND, B, LIST>);
   set((const void *)pair_kernel<T, 1, 1, -1, KIND, B, LIST>);
   set((const void *)pair_kernel<T, 1, 1, 1, KIND, B, LIST>);
+  return e;
 }
 
+// 0: the kernel cannot run on the current device
 template <typename T, bool B, int LIST>
 int resident_ctas() {
   int dev = 0, sms = 0, per = 0;
@@ -1311,8 +1315,6 @@ int resident_ctas() {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, pair_kernel<T, 1, 1, 1, 1, B, LIST>, TT,
                                                 Ring<T, LIST>::SMEM);
-  if (per < 1) per = 1;
-  if (sms < 1) sms = 1;
   return per * sms;
 }
 
@@ -1322,7 +1324,7 @@ typedef void (*LaunchFn)(const Plan &, const Maps *, const StageArgs &, const Wo
                          cudaStream_t);
 struct Entry {
   LaunchFn launch[2];     // [batched]
-  void (*attrs)();        // both forms
+  cudaError_t (*attrs)(); // both forms
   int (*resident[2])();   // [batched] CTAs resident on the device
 };
 #define CGFD_PAIR_DECL(E) \
@@ -1335,7 +1337,10 @@ CGFD_PAIR_DECL(b)
 template <typename T, int KIND, int LIST>
 Entry make_entry() {
   return Entry{{launch_dirs<T, KIND, false, LIST>, launch_dirs<T, KIND, true, LIST>},
-               [] { set_attrs<T, KIND, false, LIST>(); set_attrs<T, KIND, true, LIST>(); },
+               [] {
+                 const cudaError_t e = set_attrs<T, KIND, false, LIST>();
+                 return e == cudaSuccess ? set_attrs<T, KIND, true, LIST>() : e;
+               },
                {[]() -> int { if constexpr (KIND == 1) return resident_ctas<T, false, LIST>(); else return 0; },
                 []() -> int { if constexpr (KIND == 1) return resident_ctas<T, true, LIST>(); else return 0; }}};
 }

@@ -24,7 +24,7 @@ struct Launch {
   int list;                 // the kernel's (stage_pair_impl.cuh)
   std::vector<int4> items;  // the list it walks
 };
-constexpr int DEVICES = 2, SMS = 148;
+constexpr int DEVICES = 3, SMS = 148;
 int device = 0;
 cudaError_t last = cudaSuccess;
 std::map<std::string, std::pair<int, int>> fail;  // call -> calls to pass, then the error

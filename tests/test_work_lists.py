@@ -87,3 +87,24 @@ def test_failed_work_shape_leaves_the_lists_in_use(fake, call, nth):
     s.step_timed(1, per_stage=True)  # the launch of a freed list fails
     assert _launched(fake) == before
     s.close()
+
+
+@pytest.mark.parametrize("kernel,storage", [(cgfd.KERNEL_FUSED, cgfd.STORE_F32),
+                                            (cgfd.KERNEL_FUSED, cgfd.STORE_F16),
+                                            (cgfd.KERNEL_FUSED, cgfd.STORE_BF16),
+                                            (cgfd.KERNEL_SCALAR, cgfd.STORE_F32)])
+def test_kernel_attributes_are_set_on_every_device(fake, kernel, storage):
+    """The dynamic shared memory of the tiled kernels is opted into per device:
+    solvers of one process on several devices all launch.  An opt-in that fails
+    is reported by the solver's creation and tried again by the next."""
+    m = _model()
+    for device in (0, 1, 2):
+        if device == 2:
+            fake.fake_fail(b"cudaFuncSetAttribute", 5, cudaErrorMemoryAllocation)
+            with pytest.raises(cgfd.CgfdError, match="out of memory"):
+                cgfd.Solver(m.desc(kernel=kernel, storage=storage, device=device))
+            assert fake.fake_last() == 0
+        s = cgfd.Solver(m.desc(kernel=kernel, storage=storage, device=device))
+        m.load(s)
+        s.prepare()  # captures every launch
+        s.close()
