@@ -184,8 +184,8 @@ std::vector<Tile> y_tiles(const Geom &g) {
 }
 
 // Work items of one or more models, in two lists: lean items (no PML cell, no
-// cell outside the grid; `plain` models only) and general ones.  Item: tile
-// origin, z range, 2 * model + part.  The bottom PML layer is a z-chunk of
+// cell outside the grid; `plain` models only) and general ones (part 0, both
+// parts' launches walk them).  The bottom PML layer is a z-chunk of
 // its own (in general columns when it has >= 8 planes), the rest is cut into
 // pieces.  Order: the most expensive first (estimated cost: planes x sum over
 // the tile's valid columns of (1 + pml_weight x number of PML directions)), so
@@ -194,7 +194,7 @@ std::vector<Tile> y_tiles(const Geom &g) {
 // L2, and the two parts of a tile follow one another.
 std::vector<int4> build_items(const std::vector<Geom> &gs, const std::vector<char> &plain,
                               bool lean, int G, const WorkParams &wp, int *zchunk) {
-  struct It { int4 v; double cost; };
+  struct It { Item v; double cost; };
   struct Col { int i0, j0, z0, z1, mdl; double w; bool cut; };
   std::vector<Col> cols;  // columns with their z range, to be cut into pieces
   double planes = 0;
@@ -252,23 +252,22 @@ std::vector<int4> build_items(const std::vector<Geom> &gs, const std::vector<cha
     for (int q = 0; q < pieces; ++q) {
       const int a0 = c.z0 + (int)((long)n * q / pieces);
       const int a1 = c.z0 + (int)((long)n * (q + 1) / pieces);
-      items.push_back({make_int4(c.i0, c.j0, a0 | (a1 << 16), c.mdl), c.w * (a1 - a0)});
+      items.push_back({Item{c.i0, c.j0, a0, a1, c.mdl, 0}, c.w * (a1 - a0)});
     }
   }
   // z-chunks of a class together: columns were cut one by one
   std::stable_sort(items.begin(), items.end(), [](const It &x, const It &y) {
     if (x.cost != y.cost) return x.cost > y.cost;
-    if (x.v.w != y.v.w) return x.v.w < y.v.w;
-    return (x.v.z & 0xffff) < (y.v.z & 0xffff);
+    if (x.v.model != y.v.model) return x.v.model < y.v.model;
+    return x.v.z0 < y.v.z0;
   });
   std::vector<int4> hv;
   hv.reserve(2 * items.size());
-  auto push = [&](int4 v) {
-    v.w *= 2;
-    hv.push_back(v);  // PART_VEL
-    if (!lean) return;
-    v.w += 1;
-    hv.push_back(v);  // PART_STR
+  auto push = [&](Item v) {
+    for (int part : {PART_VEL, PART_STR}) {
+      v.part = part;
+      if (lean || part == PART_VEL) hv.push_back(pack_item(v));
+    }
   };
   // guided end: the last items (the cheapest, one per resident CTA) become
   // short chunks, ordered piece by piece (the first piece of every cut item,
@@ -277,22 +276,22 @@ std::vector<int4> build_items(const std::vector<Geom> &gs, const std::vector<cha
   size_t ncut = 0;
   if (wp.tail_chunk >= 4) {
     while (parts * ncut < (size_t)G && ncut < items.size()) {
-      const int4 v = items[items.size() - 1 - ncut].v;
-      if ((v.z >> 16) - (v.z & 0xffff) < 2 * wp.tail_chunk) break;
+      const Item &v = items[items.size() - 1 - ncut].v;
+      if (v.z1 - v.z0 < 2 * wp.tail_chunk) break;
       ++ncut;
     }
   }
   const size_t keep = items.size() - ncut;
   for (size_t q = 0; q < keep; ++q) push(items[q].v);
-  std::vector<std::vector<int4>> pieces(ncut);
+  std::vector<std::vector<Item>> pieces(ncut);
   size_t maxp = 0;
   for (size_t q = 0; q < ncut; ++q) {
-    const int4 v = items[keep + q].v;
-    const int z0 = v.z & 0xffff, z1 = v.z >> 16, np = (z1 - z0) / wp.tail_chunk;
+    Item v = items[keep + q].v;
+    const int z0 = v.z0, n = v.z1 - z0, np = n / wp.tail_chunk;
     for (int t = 0; t < np; ++t) {
-      const int a0 = z0 + (int)((long)(z1 - z0) * t / np);
-      const int a1 = z0 + (int)((long)(z1 - z0) * (t + 1) / np);
-      pieces[q].push_back(make_int4(v.x, v.y, a0 | (a1 << 16), v.w));
+      v.z0 = z0 + (int)((long)n * t / np);
+      v.z1 = z0 + (int)((long)n * (t + 1) / np);
+      pieces[q].push_back(v);
     }
     maxp = std::max(maxp, pieces[q].size());
   }
@@ -443,7 +442,7 @@ void launch_stage_pair(const void *plan, const StageArgs &a, int in_set, int *er
 
 void *pair_create_batch_plan(int n, const Geom *gs, void *const *sets, const float *const *media,
                              const float *const *metric, float *const *aux, int elem) {
-  if (!set_attrs_of(elem)) return nullptr;
+  if (n > ITEM_MODELS || !set_attrs_of(elem)) return nullptr;
   Plan *pl = new (std::nothrow) Plan();
   if (!pl) return nullptr;
   pl->elem = elem;

@@ -154,11 +154,32 @@ struct Maps {
   CUtensorMap aux[3][3];  // [direction][ain, afw, ta], box {32, 8, 1, NS}
 };
 
-// Work list of a launch: items {i0, j0, z0 | z1 << 16, model} (tile
-// origin, z range, model of a batch), ordered by decreasing estimated cost;
-// CTAs take them in order from an atomic counter (reset before every
-// launch), so expensive PML items start first and the cheap interior items
-// fill the tail.  A batched launch reads each model's stage arguments and
+// A work item: the planes [z0, z1) of the tile of columns at (i0, j0).  Packed
+// into one 128-bit load: {i0, j0, z0, z1}, planes in 21 bits (grid sides reach
+// 2^20 cells), the 11 above them hold 2 * model + part in two halves.
+struct Item {
+  int i0, j0, z0, z1, model, part;
+};
+constexpr int ITEM_Z_BITS = 21, ITEM_MODELS = 1 << (2 * (32 - ITEM_Z_BITS) - 1);
+__host__ __device__ inline int4 pack_item(const Item &t) {
+  const unsigned mp = 2u * (unsigned)t.model + (unsigned)t.part, hi = 32 - ITEM_Z_BITS;
+  int4 v;
+  v.x = t.i0;
+  v.y = t.j0;
+  v.z = (int)((unsigned)t.z0 | (mp & ((1u << hi) - 1)) << ITEM_Z_BITS);
+  v.w = (int)((unsigned)t.z1 | mp >> hi << ITEM_Z_BITS);
+  return v;
+}
+__host__ __device__ inline Item unpack_item(const int4 &v) {
+  const unsigned z = (unsigned)v.z, w = (unsigned)v.w, mask = (1u << ITEM_Z_BITS) - 1;
+  const unsigned mp = z >> ITEM_Z_BITS | w >> ITEM_Z_BITS << (32 - ITEM_Z_BITS);
+  return Item{v.x, v.y, (int)(z & mask), (int)(w & mask), (int)(mp >> 1), (int)(mp & 1)};
+}
+
+// Work list of a launch: packed items ordered by decreasing estimated cost;
+// CTAs take them in order from an atomic counter (reset by the last CTA of the
+// launch before), so expensive PML items start first and the cheap interior
+// items fill the tail.  A batched launch reads each model's stage arguments and
 // tensor maps from the device arrays bargs / bmaps (one entry per model).
 struct Work {
   const int4 *items[2];  // general, lean
@@ -943,7 +964,7 @@ struct RingState {
 // cell of the tile valid.
 template <typename T, int PART, int X, int Y, int Z, int KIND, bool LEAN>
 __device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const Work &wk,
-                                      const bool (&aux_on)[3], const int4 it, bool withhold_item,
+                                      const bool (&aux_on)[3], const Item &it, bool withhold_item,
                                       unsigned char *ring, uint64_t *bars, RingState &rs,
                                       volatile int *abort_flag) {
   using S = Slot<T, PART>;
@@ -969,9 +990,9 @@ __device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const W
   auto zz_of = [&](int p) { return flat ? 1.f : (p < A.zu_end ? A.zzp[p] : 0.f); };
   const float rh = 1.f / A.h;
   const int zlo = LFD + g.nabs[4], zhi = g.nk + LFD - g.nabs[5];  // z interior [zlo, zhi)
-  const int i0 = it.x, j0 = it.y, z0 = it.z;
+  const int i0 = it.i0, j0 = it.j0, z0 = it.z0;
   // the traction image owns the top three layers' velocities
-  const int z1 = (LEAN && PART == PART_VEL) ? min(it.w, g.top - 2) : it.w;
+  const int z1 = (LEAN && PART == PART_VEL) ? min(it.z1, g.top - 2) : it.z1;
   const int n = z1 - z0;                   // planes computed
   if (n <= 0) return;
   const int zf = (DIR > 0) ? z0 : z1 - 1;  // first plane in march order
@@ -1195,8 +1216,8 @@ __global__ void __launch_bounds__(TT, (Ring<T, LIST>::CTAS))
       __syncthreads();
       const int cur = s_next;
       if (cur >= wk.nitems[LEAN]) break;  // CTA-uniform
-      const int4 it4 = wk.items[LEAN][cur];
-      const int part = LEAN ? it4.w & 1 : LIST, model = B ? it4.w >> 1 : 0;
+      const Item it = unpack_item(wk.items[LEAN][cur]);
+      const int part = LEAN ? it.part : LIST, model = B ? it.model : 0;
       // a batched launch reads the item's model's stage arguments in place
       // (global memory, read-only during the launch).  Copied per item into a
       // __shared__ StageArgs and read from there, the 16-bit batched stages
@@ -1208,7 +1229,6 @@ __global__ void __launch_bounds__(TT, (Ring<T, LIST>::CTAS))
       const bool aux_on[3] = {B ? A.ain[0] != nullptr : wk.has_aux[0] != 0,
                               B ? A.ain[1] != nullptr : wk.has_aux[1] != 0,
                               B ? A.ain[2] != nullptr : wk.has_aux[2] != 0};
-      const int4 it = make_int4(it4.x, it4.y, it4.z & 0xffff, it4.z >> 16);
       if (LIST == GEN_VEL || (LEAN && part == PART_VEL))
         march<T, PART_VEL, X, Y, Z, KIND, LEAN>(A, B ? wk.bmaps[model] : maps_v, wk, aux_on, it,
                                                 cur == 0, ring, bars, rs, &abort_flag);

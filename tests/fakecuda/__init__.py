@@ -9,6 +9,8 @@ import os
 import shutil
 import subprocess
 
+import numpy as np
+
 import cgfd
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -43,10 +45,7 @@ def lib(path):
 
 
 def items(h, q):
-    """The items of launch q: (i0, j0, word 2, word 3)."""
-    v = (C.c_int * 4)()
-    out = []
-    for k in range(h.fake_items(q)):
-        h.fake_item(q, k, v)
-        out.append(tuple(v))
-    return out
+    """The items of launch q, rows of i0, j0, z0, z1, model, part."""
+    v = np.zeros((h.fake_items(q), 6), np.int32)
+    h.fake_get_items(q, v.ctypes.data_as(C.POINTER(C.c_int)))
+    return v

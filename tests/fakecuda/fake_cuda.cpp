@@ -17,6 +17,7 @@
 
 // the paired stage kernels' argument (paired_work.cu)
 extern "C" const int4 *paired_items(const void *work, int list, int *n);
+extern "C" void paired_item(const int4 *packed, int *v);
 
 namespace {
 
@@ -29,6 +30,7 @@ int device = 0;
 cudaError_t last = cudaSuccess;
 std::map<std::string, std::pair<int, int>> fail;  // call -> calls to pass, then the error
 std::map<const void *, size_t> memory;
+std::set<const void *> fresh;  // allocated (zeros) and not yet written
 std::set<std::pair<int, const void *>> attrs;
 std::vector<Launch> launches;
 std::map<const void *, std::string> names;  // kernels
@@ -77,11 +79,14 @@ void fake_reset() {
 void fake_fail(const char *call, int pass, int e) { fail[call] = {pass, e}; }
 int fake_blocks() { return (int)memory.size(); }
 void fake_clear_launches() { launches.clear(); }
-// launches of the paired stage kernels so far: list and items (item k's four words)
+// launches of the paired stage kernels so far: list and items
+// (i0, j0, z0, z1, model, part of each)
 int fake_launches() { return (int)launches.size(); }
 int fake_list(int q) { return launches[q].list; }
 int fake_items(int q) { return (int)launches[q].items.size(); }
-void fake_item(int q, int k, int *v) { std::memcpy(v, &launches[q].items[k], 16); }
+void fake_get_items(int q, int *v) {
+  for (const int4 &t : launches[q].items) paired_item(&t, v), v += 6;
+}
 // the last (unread) error, as cudaPeekAtLastError
 int fake_last() { return (int)last; }
 
@@ -126,6 +131,7 @@ cudaError_t cudaMalloc(void **p, size_t n) {
   void *q = std::calloc(1, n ? n : 1);
   if (!q) return ret(cudaErrorMemoryAllocation);
   memory[q] = n;
+  fresh.insert(q);
   *p = q;
   return cudaSuccess;
 }
@@ -136,21 +142,25 @@ cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
 cudaError_t cudaFree(void *p) {
   if (!p) return cudaSuccess;
   if (!memory.erase(p)) return ret(cudaErrorInvalidValue);  // not (or no longer) allocated
+  fresh.erase(p);
   std::free(p);
   return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
   if (const cudaError_t e = planted("cudaMemcpy")) return ret(e);
+  fresh.erase(d);
   std::memcpy(d, s, n);
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind,
                                    cudaStream_t) {
+  fresh.erase(d);
   std::memcpy(d, s, n);
   return cudaSuccess;
 }
 cudaError_t cudaMemset(void *d, int v, size_t n) {
-  std::memset(d, v, n);
+  // the first one of a block has nothing to do (and leaves its pages untouched)
+  if (v != 0 || !fresh.erase(d)) std::memset(d, v, n);
   return cudaSuccess;
 }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {

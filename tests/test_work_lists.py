@@ -1,5 +1,7 @@
 """The stage kernels' work lists and the launch plan around them, on a CUDA
 runtime that lives on the host (tests/fakecuda): no GPU, no kernel runs."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -38,7 +40,7 @@ def _launched(h):
     out = {}
     for q in range(h.fake_launches()):
         it = fakecuda.items(h, q)
-        assert out.setdefault(h.fake_list(q), it) == it
+        assert np.array_equal(out.setdefault(h.fake_list(q), it), it)
     return out
 
 
@@ -85,7 +87,8 @@ def test_failed_work_shape_leaves_the_lists_in_use(fake, call, nth):
     assert s.work_shape == shape and fake.fake_last() == 0
     fake.fake_clear_launches()
     s.step_timed(1, per_stage=True)  # the launch of a freed list fails
-    assert _launched(fake) == before
+    after = _launched(fake)
+    assert set(after) == set(before) and all(np.array_equal(after[k], before[k]) for k in after)
     s.close()
 
 
@@ -108,3 +111,74 @@ def test_kernel_attributes_are_set_on_every_device(fake, kernel, storage):
         m.load(s)
         s.prepare()  # captures every launch
         s.close()
+
+
+TILE_X, TILE_Y, LFD = 32, 8, 3
+GRIDS = [  # ni, nj, nk, nabs
+    (96, 40, 24, (8, 8, 8, 8, 8, 0)),
+    (64, 16, 12, (0, 0, 0, 0, 0, 0)),
+    (101, 27, 19, (32, 5, 3, 1, 4, 0)),
+    (100, 9, 20, (1, 35, 0, 0, 9, 0)),
+    (40, 30, 13, (4, 4, 4, 4, 6, 0)),
+    (1, 1, 4, (0, 0, 0, 0, 0, 0)),
+    (200, 300, 4, (20, 20, 20, 20, 2, 0)),
+    (40, 12, 33000, (4, 4, 0, 0, 8, 0)),  # planes past 2^15
+    (32, 8, 70000, (0, 0, 0, 0, 0, 0)),  # and past 2^16
+]
+
+
+def _covered(it, model):
+    """How often the items of one model and part compute each cell."""
+    ni, nj, nk, nabs = model
+    n = np.zeros((nk, nj, ni), np.int8)
+    for i0, j0, z0, z1 in it[:, :4]:
+        assert i0 % TILE_X == 0 and i0 < ni and LFD <= z0 < z1 <= nk + LFD
+        n[z0 - LFD:z1 - LFD, max(j0, 0):max(j0 + TILE_Y, 0), i0:i0 + TILE_X] += 1
+    return n
+
+
+@pytest.mark.parametrize("plain", [True, False], ids=["plain", "not_plain"])
+@pytest.mark.parametrize("grids", [[g] for g in GRIDS] + [GRIDS[:5]],
+                         ids=["x".join(map(str, g[:3])) for g in GRIDS] + ["batch"])
+def test_items_cover_every_cell_once(fake, grids, plain):
+    """Every cell is an item's of each part exactly once; lean items hold cells
+    of the grid outside the layers only, and where a model is deep enough they
+    hold every whole tile of those."""
+    descs = [cgfd.Desc(ni=ni, nj=nj, nk=nk, steph=100.0, stept=0.005, nt=4,
+                       con_index=nk // 2 + LFD, hybrid_grid=1, nabs=(C.c_int * 6)(*nabs))
+             for ni, nj, nk, nabs in grids]
+    b = cgfd.Batch(descs) if len(grids) > 1 else None
+    solvers = b.models if b else [cgfd.Solver(descs[0])]
+    for s, (ni, nj, nk, _) in zip(solvers, grids):
+        shape = (ni + 6, nj + 6, nk + 6)
+        one, zero = np.ones(shape), np.zeros(shape)
+        s.upload_metric(zero, zero, one, one)
+        s.upload_media(*(np.full(shape, v, np.float32) for v in (6000.0, 3464.0, 2670.0)))
+        prof = [[np.full(n, v) for n in shape] for v in (0.0, 1.0, 0.0)]
+        if not plain:
+            prof[1][2][nk // 2 + LFD] = 1.25
+        s.upload_pml(*prof)
+    if b:  # not the members' own launches
+        for s in solvers:
+            s.prepare()
+        fake.fake_clear_launches()
+    (b or solvers[0]).prepare()
+    lists = _launched(fake)
+    for k, g in enumerate(grids):
+        ni, nj, nk, nabs = g
+        of = {q: it[it[:, 4] == k] for q, it in lists.items()}
+        none = np.zeros((0, 6), np.int32)
+        lean = of.get(fakecuda.LEAN, none)
+        general = of.get(fakecuda.GEN_VEL, none)
+        assert np.array_equal(general, of.get(fakecuda.GEN_STR, none))
+        parts = [_covered(lean[lean[:, 5] == p], g) for p in (0, 1)]
+        assert np.array_equal(*parts)
+        assert np.all(parts[0] + _covered(general, g) == 1)
+        for i0, j0, z0, _ in lean[:, :4]:
+            assert nabs[0] <= i0 <= ni - nabs[1] - TILE_X
+            assert nabs[2] <= j0 <= nj - nabs[3] - TILE_Y and z0 - LFD >= nabs[4]
+        whole = max(sum(nabs[0] <= i <= ni - nabs[1] - TILE_X for i in range(0, ni, TILE_X)), 0) * \
+            ((nj - nabs[2] - nabs[3]) // TILE_Y) * (nk - nabs[4])
+        want = whole * TILE_X * TILE_Y if plain and nk - nabs[4] >= 8 else 0
+        assert parts[0].sum(dtype=np.int64) == want
+    (b or solvers[0]).close()
