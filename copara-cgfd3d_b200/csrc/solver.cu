@@ -554,28 +554,29 @@ void free_all(cgfd_solver *h) {
 // solver (grown, never shrunk, freed with it), larger ones live for the call.
 constexpr size_t STAGE_KEEP = 64u << 20;
 struct Stage {
-  cgfd_solver *h;
   float *p = nullptr;
   bool own = false;
-  Stage(cgfd_solver *hh, size_t n) : h(hh) {
+  cudaError_t e = cudaSuccess;  // why p is null
+  Stage(cgfd_solver *h, size_t n) {
     const size_t b = n * sizeof(float);
-    if (b > STAGE_KEEP) {
-      own = cudaMalloc(&p, b) == cudaSuccess;
-      if (!own) p = nullptr, cudaGetLastError();
-      return;
-    }
-    if (b > h->stage_cap) {
-      cudaFree(h->stage);
-      h->stage = nullptr;
-      h->stage_cap = 0;
-      if (cudaMalloc(&h->stage, b) != cudaSuccess) {
+    own = b > STAGE_KEEP;
+    if (own || b > h->stage_cap) {
+      if (!own) {
+        cudaFree(h->stage);
         h->stage = nullptr;
-        cudaGetLastError();
+        h->stage_cap = 0;
+      }
+      e = cudaMalloc(&p, b);
+      if (e != cudaSuccess) {
+        p = nullptr;
         return;
       }
-      h->stage_cap = b;
+      if (!own) {
+        h->stage = p;
+        h->stage_cap = b;
+      }
     }
-    p = h->stage;
+    if (!own) p = h->stage;
   }
   Stage(const Stage &) = delete;
   ~Stage() {
@@ -594,7 +595,7 @@ int upload_ref(cgfd_solver *h, const float *host, void *dst, int elem = ELEM_F32
   const long n = ref_n(h);
   Stage stage(h, n);
   float *const tmp = stage.p;
-  if (!tmp) return cuda_fail(h, cudaErrorMemoryAllocation, "upload");
+  if (!tmp) return cuda_fail(h, stage.e, "upload");
   cudaError_t e = cudaMemcpyAsync(tmp, host, n * sizeof(float), cudaMemcpyHostToDevice, h->st);
   if (e == cudaSuccess) {
     const int nx = h->d.ni + 6, ny = h->d.nj + 6, nz = h->d.nk + 6;
@@ -653,7 +654,7 @@ int upload_fields(cgfd_solver *h, int count, Fill &&fill, float *const *dst) {
   }
   Stage stage(h, n);
   float *const tmp = stage.p;
-  if (!tmp) return cuda_fail(h, cudaErrorMemoryAllocation, "upload");
+  if (!tmp) return cuda_fail(h, stage.e, "upload");
   const int nx = h->d.ni + 6, ny = h->d.nj + 6, nz = h->d.nk + 6;
   cudaError_t e = cudaSuccess;
   int c = 0;
@@ -682,7 +683,7 @@ int download_ref(cgfd_solver *h, const void *src, float *host, int elem = ELEM_F
   const long n = ref_n(h);
   Stage stage(h, n);
   float *const tmp = stage.p;
-  if (!tmp) return cuda_fail(h, cudaErrorMemoryAllocation, "download");
+  if (!tmp) return cuda_fail(h, stage.e, "download");
   const int nx = h->d.ni + 6, ny = h->d.nj + 6, nz = h->d.nk + 6;
   if (elem == ELEM_F16)
     to_reference_kernel<<<592, 256, 0, h->st>>>((const __half *)src, tmp, h->g, nx, ny, nz, sc);
@@ -2666,7 +2667,7 @@ int cgfd_get_snapshot(cgfd_solver *h, int set, const int *start, const int *coun
   const int parts = add_fw ? 2 : 1;
   Stage stage(h, parts * n);
   float *const tmp = stage.p;
-  if (!tmp) return cuda_fail(h, cudaErrorMemoryAllocation, "snapshot");
+  if (!tmp) return cuda_fail(h, stage.e, "snapshot");
   ScaleSet sc;
   for (int c = 0; c < NCOMP; ++c) sc.sc[c] = std::ldexp(1.f, h->sexp[c]);
   const int3 st3 = make_int3(start[0], start[1], start[2]);

@@ -8,6 +8,8 @@ pre-processing, and the C ABI's symbol table.
 import os
 import sys
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 for p in (os.path.join(ROOT, "copara-cgfd3d_b200", "python"), os.path.join(ROOT, "oracle"),
           os.path.join(ROOT, "tests"), os.path.join(ROOT, "tests", "golden")):
@@ -18,3 +20,21 @@ for p in (os.path.join(ROOT, "copara-cgfd3d_b200", "python"), os.path.join(ROOT,
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200) and the built libraries")
     config.addinivalue_line("markers", "slow: longer full-size parity runs")
+
+
+@pytest.fixture(scope="session")
+def fake_lib(tmp_path_factory):
+    import fakecuda
+    path = fakecuda.build(str(tmp_path_factory.mktemp("fakecuda")))
+    if path is None:
+        pytest.skip("nvcc and g++ are needed")
+    return fakecuda.lib(path)
+
+
+@pytest.fixture
+def fake(fake_lib, monkeypatch):
+    """The library on a CUDA runtime that lives on the host (tests/fakecuda)."""
+    import cgfd
+    fake_lib.fake_reset()
+    monkeypatch.setattr(cgfd, "_lib", fake_lib)
+    return fake_lib

@@ -109,9 +109,10 @@ cudaError_t __cudaPopCallConfiguration(dim3 *grid, dim3 *block, size_t *smem, vo
   return cudaSuccess;
 }
 const char *cudaGetErrorString(cudaError_t e) {
-  return e == cudaErrorMemoryAllocation ? "out of memory"
-         : e == cudaSuccess             ? "no error"
-                                        : "planted error";
+  return e == cudaSuccess                ? "no error"
+         : e == cudaErrorMemoryAllocation ? "out of memory"
+         : e == cudaErrorIllegalAddress   ? "an illegal memory access"
+                                          : "another error";
 }
 cudaError_t cudaGetDeviceCount(int *n) { *n = DEVICES; return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = device; return cudaSuccess; }

@@ -12,21 +12,6 @@ import models
 cudaErrorMemoryAllocation = 2
 
 
-@pytest.fixture(scope="module")
-def fake_lib(tmp_path_factory):
-    path = fakecuda.build(str(tmp_path_factory.mktemp("fakecuda")))
-    if path is None:
-        pytest.skip("nvcc and g++ are needed")
-    return fakecuda.lib(path)
-
-
-@pytest.fixture
-def fake(fake_lib, monkeypatch):
-    fake_lib.fake_reset()
-    monkeypatch.setattr(cgfd, "_lib", fake_lib)
-    return fake_lib
-
-
 def _model(ni=96, nj=40, nk=24, nabs=(8, 8, 8, 8, 8, 0)):
     return models.gaussian_hill(ni=ni, nj=nj, nk=nk, nt=4, dz_top=60.0, dz_bot=120.0,
                                 hill_h=200.0, hill_w=600.0, con_depth=400.0, src_depth=300.0,
