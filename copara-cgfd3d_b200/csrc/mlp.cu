@@ -645,6 +645,7 @@ struct GradBuffers {
   float *x = nullptr, *t = nullptr, *partial = nullptr, *out = nullptr;
   size_t ncap = 0;
   int nblocks = 0;
+  bool ready = false;  // all but x and t
 };
 std::mutex g_grad_lock;
 std::vector<GradBuffers> g_grad;
@@ -669,15 +670,16 @@ extern "C" int cgfd_mlp_gradient(const void *weights_fp16, const float *x, const
   }
   if ((int)g_grad.size() <= dev) g_grad.resize(dev + 1);
   GradBuffers &B = g_grad[dev];
-  if (!B.w) {
-    B.nblocks = sms > 0 ? sms : 148;
-    e = cudaMalloc(&B.w, NPAR * sizeof(__half));
-    if (e == cudaSuccess)
+  if (!B.ready) {  // (also after a first call that failed part of the way)
+    B.nblocks = sms;
+    if (!B.w) e = cudaMalloc(&B.w, NPAR * sizeof(__half));
+    if (e == cudaSuccess && !B.partial)
       e = cudaMalloc(&B.partial, (size_t)B.nblocks * (NPAR + 1) * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&B.out, (NPAR + 1) * sizeof(float));
+    if (e == cudaSuccess && !B.out) e = cudaMalloc(&B.out, (NPAR + 1) * sizeof(float));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)GRAD_SMEM);
+    B.ready = e == cudaSuccess;
   }
   if (e == cudaSuccess && (size_t)n > B.ncap) {
     cudaFree(B.x);
@@ -701,6 +703,7 @@ extern "C" int cgfd_mlp_gradient(const void *weights_fp16, const float *x, const
   if (e == cudaSuccess) e = cudaMemcpy(grad, B.out, NPAR * sizeof(float), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(loss, B.out + NPAR, sizeof(float), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     set_global_error(cudaGetErrorString(e));
     return CGFD_ERR_CUDA;
   }

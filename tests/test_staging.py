@@ -1,6 +1,6 @@
-"""Device staging of uploads, downloads and snapshots (kept with the solver up to
-64 MB, per call above), on a CUDA runtime that lives on the host
-(tests/fakecuda)."""
+"""Device buffers kept between calls -- the staging of uploads, downloads and
+snapshots (with the solver up to 64 MB, per call above) and the training
+gradient's -- on a CUDA runtime that lives on the host (tests/fakecuda)."""
 import numpy as np
 import pytest
 
@@ -37,3 +37,22 @@ def test_failed_staging_reports_its_cause(fake, call, error, text, side):
     CALLS[call](s)
     s.close()
     assert fake.fake_blocks() == blocks
+
+
+@pytest.mark.parametrize("what,nth", [(b"cudaMalloc", k) for k in range(5)] +
+                         [(b"cudaFuncSetAttribute", 0)])
+def test_failed_gradient_buffers_are_tried_again(fake, what, nth):
+    """A first gradient call on a device that fails part of the way through its
+    buffers leaves the next one to finish them (its launch would be refused
+    without them)."""
+    w = np.zeros(cgfd.MLP_PARAMS, np.float16)
+    x, t = np.zeros((300, 45), np.float32), np.zeros((300, 9), np.float32)
+    fake.cudaSetDevice(10 + nth + 10 * (what != b"cudaMalloc"))  # one without buffers yet
+    blocks = fake.fake_blocks()
+    fake.fake_fail(what, nth, cudaErrorMemoryAllocation)
+    with pytest.raises(cgfd.CgfdError, match="out of memory"):
+        cgfd.mlp_gradient(w, x, t)
+    assert fake.fake_last() == 0
+    cgfd.mlp_gradient(w, x, t)
+    cgfd.mlp_gradient(w, x, t)
+    assert fake.fake_blocks() == blocks + 5
