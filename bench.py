@@ -50,7 +50,7 @@ def parse():
                         "single models; batch64 tunes only when asked)")
     p.add_argument("--no-autotune", dest="autotune", action="store_false")
     p.add_argument("--work-shape", default=None, metavar="ITEMS,CHUNK,PMLW",
-                   help="single models: use this work shape (items per resident CTA, minimum "
+                   help="single models: use this work shape (items per resident CTA, "
                         "z-chunk, PML cost weight; a line's work_shape) instead of tuning")
     p.add_argument("--tune-batch", action="store_true",
                    help="batch64: tune the work list and launch shape before timing")

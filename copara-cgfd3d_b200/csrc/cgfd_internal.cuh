@@ -190,9 +190,9 @@ int fused_plan_info(const void *plan, int *zchunk, int *grid_vel, int *grid_str)
 // The paired kernels (two x-adjacent cells per thread, stage_pair.cu); aux
 // holds the three directions' auxiliary arrays (null: no PML there).
 // Shape of the paired kernels' work list (the autotuner's knobs): about
-// items_per_cta items per resident CTA, z-chunks of at least min_chunk
-// planes, PML columns weighted (1 + pml_weight per direction) in the cost
-// order.
+// items_per_cta items per resident CTA, z-chunks of about min_chunk planes at
+// the least (shorter where those would leave CTAs without an item), PML columns
+// weighted (1 + pml_weight per direction) in the cost order.
 #ifndef CGFD_TAIL_CHUNK
 #define CGFD_TAIL_CHUNK 8
 #endif
@@ -214,6 +214,8 @@ bool pair_set_plain(void *plan, const char *plain);
 // restores the defaults
 bool pair_set_wait_test(void *plan, double wait_s, int withhold);
 WorkParams pair_get_work(const void *plan);
+// a number that stands for the plan's current lists (shapes may share them)
+unsigned long long pair_work_id(const void *plan);
 void *pair_create_plan(const Geom &g, int elem, void *const sets[4], const float *media,
                        const float *metric, float *const aux[3]);
 void pair_destroy_plan(void *plan);

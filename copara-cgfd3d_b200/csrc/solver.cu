@@ -24,6 +24,7 @@
 #include <exception>
 #include <limits>
 #include <memory>
+#include <set>
 #include <string>
 #include <thread>
 #include <vector>
@@ -2067,11 +2068,13 @@ int cgfd_autotune(cgfd_solver *h, int steps, float *best_ms) {
   if (st) return st;
   float best = 1e30f;
   WorkParams bestp = pair_get_work(h->plan);
+  std::set<unsigned long long> tried;  // the lists
   for (const WorkParams &wp : tuning_candidates(bestp)) {
     if (!pair_set_work(h->plan, wp)) {
       list_error();
       continue;
     }
+    if (!tried.insert(pair_work_id(h->plan)).second) continue;
     h->graphs_ok = false;
     st = build_graphs(h);
     if (st) break;
@@ -2514,11 +2517,13 @@ int cgfd_batch_autotune(cgfd_batch *b, int steps, float *best_ms) {
   }
   float best = 1e30f;
   WorkParams bestp = pair_get_work(b->plan);
+  std::set<unsigned long long> tried;  // the lists
   for (const WorkParams &wp : tuning_candidates(bestp)) {
     if (!pair_set_work(b->plan, wp)) {
       list_error();
       continue;
     }
+    if (!tried.insert(pair_work_id(b->plan)).second) continue;
     b->ready = false;
     st = batch_build(b);
     if (st) break;

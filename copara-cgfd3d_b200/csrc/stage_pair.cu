@@ -70,8 +70,8 @@ bool aux_map(CUtensorMap *m, const Geom &g, int d, const float *base, int bc) {
 using namespace pair;
 
 bool pair_supported(const Geom &g) {
-  // tile boxes start on 16-byte boundaries (XO and i0 multiples of 4, px of
-  // 32) and every z-chunk has at least 4 planes
+  // tile boxes start on 16-byte boundaries (XO and i0 multiples of 4, px of 32);
+  // the free surface and the two layers below it are distinct planes
   return (XO % 4) == 0 && XO >= 4 && g.px % 32 == 0 && g.nk >= 4;
 }
 
@@ -232,8 +232,8 @@ std::vector<int4> build_items(const std::vector<Geom> &gs, const std::vector<cha
       }
   }
   if (cols.empty()) return {};
-  // chunk length: about items_per_cta items per resident CTA, at least
-  // min_chunk planes; but where that leaves resident CTAs without an item, as
+  // chunk length: about items_per_cta items per resident CTA, min_chunk planes at
+  // the least; but where that leaves resident CTAs without an item, as
   // many planes as share the work out over all of them, down to one (the stage
   // then takes a few planes' latency: 28x24x20 cells 103 us per step with
   // chunks of at least 4 planes, 73 with 2, 60 with 1; 62x54x40 cells, where
@@ -350,6 +350,10 @@ bool rebuild(Plan *pl, const WorkParams &wp, const std::vector<char> &plain) {
     hv[l] = build_items(pl->geoms, plain, l != 0,
                         l ? G[LEAN_BOTH] : std::min(G[GEN_VEL], G[GEN_STR]), wp, &zchunk);
   if (!upload_items(pl, hv, G)) return false;
+  pl->list_id = 14695981039346656037ull;  // FNV-1a over both lists
+  for (const auto &list : hv)
+    for (const int4 &v : list)
+      for (int w : {v.x, v.y, v.z, v.w}) pl->list_id = (pl->list_id ^ (unsigned)w) * 1099511628211ull;
   pl->zchunk = zchunk;
   pl->params = wp;
   pl->plain = plain;
@@ -378,6 +382,10 @@ void *pair_create_plan(const Geom &g, int elem, void *const sets[4], const float
 
 WorkParams pair_get_work(const void *plan) {
   return reinterpret_cast<const Plan *>(plan)->params;
+}
+
+unsigned long long pair_work_id(const void *plan) {
+  return reinterpret_cast<const Plan *>(plan)->list_id;
 }
 
 bool pair_set_work(void *plan, const WorkParams &wp) {

@@ -1277,6 +1277,7 @@ struct Plan {
   int zchunk = 0;              // planes of the (first model's) interior z-chunks
   int grid[NLIST];             // CTAs per launch (0: no items)
   WorkParams params;
+  unsigned long long list_id = 0;  // hash of the lists
   int nmodels = 0;             // 0: single-model plan; else a batch of nmodels
   StageArgs *d_bargs = nullptr;  // batch: [pattern * 4 + stage][model]
   Maps *d_bmaps = nullptr;       // batch: [stage][part][model]

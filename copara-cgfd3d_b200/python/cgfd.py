@@ -277,7 +277,7 @@ class Solver:
 
     @property
     def work_shape(self) -> tuple:
-        """(items per resident CTA, shortest z-chunk, PML cost weight) of the
+        """(items per resident CTA, z-chunk length, PML cost weight) of the
         work list in use (cgfd_get_work_shape; after prepare)."""
         a, b, c = C.c_int(), C.c_int(), C.c_double()
         self._chk(_lib.cgfd_get_work_shape(self._h, C.byref(a), C.byref(b), C.byref(c)))

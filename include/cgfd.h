@@ -303,8 +303,9 @@ int cgfd_mlp_gradient(const void *weights_fp16, const float *x, const float *t, 
 /* ------------------------------ autotuning ------------------------------- */
 
 /* Tries the work-list shapes of the default kernel family (items per
- * resident CTA 3/6/12/24, shortest z-chunk 12/16/24/32/48 planes, PML cost
- * weight 1/2/3, and the shape in use), times `steps` steps of each (after one
+ * resident CTA 3/6/12/24, z-chunks of 12/16/24/32/48 planes, PML cost
+ * weight 1/2/3, and the shape in use; shapes that give a list already timed
+ * are left out), times `steps` steps of each (after one
  * warm-up step), keeps the fastest and reports its time per
  * step in *ms_per_step.  The wavefields, auxiliaries, seismograms and step
  * count are saved before and restored after, so the simulation is
@@ -314,9 +315,14 @@ int cgfd_mlp_gradient(const void *weights_fp16, const float *x, const float *t, 
  * from its configuration file). */
 int cgfd_autotune(cgfd_solver *h, int steps, float *ms_per_step);
 /* The work-list shape in use (after cgfd_prepare, default kernel family):
- * items per resident CTA, shortest z-chunk in planes, PML cost weight of the
- * item order; the autotuner's choice can be read and set on another solver
- * of the same model without tuning again.  No reference counterpart. */
+ * items per resident CTA, z-chunk length in planes (min_chunk), PML cost weight
+ * of the item order; the autotuner's choice can be read and set on another solver
+ * of the same model without tuning again.  A grid large enough for items of
+ * min_chunk planes or more gets as many as items_per_cta asks for, of equal
+ * lengths near min_chunk at the least (24 planes at 16 make two of 12), and
+ * shorter ones at the end of a list; where items of min_chunk planes would leave
+ * resident CTAs without one, min_chunk gives way to the length that occupies
+ * them all (down to one plane).  No reference counterpart. */
 int cgfd_get_work_shape(cgfd_solver *h, int *items_per_cta, int *min_chunk, double *pml_weight);
 int cgfd_set_work_shape(cgfd_solver *h, int items_per_cta, int min_chunk, double pml_weight);
 

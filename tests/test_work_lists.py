@@ -167,3 +167,24 @@ def test_items_cover_every_cell_once(fake, grids, plain):
         want = whole * TILE_X * TILE_Y if plain and nk - nabs[4] >= 8 else 0
         assert parts[0].sum(dtype=np.int64) == want
     (b or solvers[0]).close()
+
+
+@pytest.mark.parametrize("grid,lists", [((28, 24, 20), 1), ((200, 160, 90), 10)])
+def test_autotuner_times_a_list_once(fake, grid, lists):
+    """On a small grid most shapes cut the same items.  (lists: at least so many
+    different ones.)"""
+    m = _model(*grid, nabs=(4, 4, 4, 4, 4, 0))
+    s = cgfd.Solver(m.desc())
+    m.load(s)
+    s.prepare()
+    fake.fake_clear_launches()
+    s.autotune(steps=1)
+    # a captured step is four stages, each with the launches of its lists; four
+    # steps are captured per shape
+    runs = [(fake.fake_list(q), fakecuda.items(fake, q).tobytes())
+            for q in range(fake.fake_launches())]
+    per = len({k for k, _ in runs})
+    shapes = [tuple(runs[k:k + per]) for k in range(0, len(runs), 4 * 4 * per)]
+    timed, chosen = shapes[:-1], shapes[-1]
+    assert len(timed) == len(set(timed)) >= lists and chosen in timed
+    s.close()
