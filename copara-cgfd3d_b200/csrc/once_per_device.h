@@ -29,4 +29,12 @@ class OncePerDevice {
   std::set<std::pair<int, int>> done_;
 };
 
+// SMs of the current device
+inline int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 }  // namespace cgfd

@@ -69,6 +69,7 @@ void *fused_create_plan(const Geom &g, float *const sets[4], const float *media,
   if (!set) return nullptr;
   Plan *pl = new (std::nothrow) Plan();
   if (!pl) return nullptr;
+  pl->sms = sm_count();
   bool ok = true;
   for (int q = 0; q < 4; ++q) {
     ok = ok && make_map(&pl->haloV[q], g, sets[q], 9, BOXX, BOXY, PartInfo<PART_VEL>::NC);
@@ -136,7 +137,7 @@ void launch_stage_fused(const void *plan, const StageArgs &a, int in_set, int *e
     launch_v2(pl, mv, a, err, s);
     launch_s2(pl, ms, a, err, s);
   }
-  launch_timg(a, s);
+  launch_timg(a, s, pl.sms);
 }
 
 int fused_plan_info(const void *plan, int *zchunk, int *grid_vel, int *grid_str) {

@@ -598,7 +598,7 @@ struct Plan {
   // pointwise boxes of V (3) and T (6) components
   CUtensorMap haloV[4], haloS[4], ctrV[4], ctrT[4];
   CUtensorMap coefV, coefS, met;
-  int zchunk, ntx, ntiles, nitems, grid[2];
+  int zchunk, ntx, ntiles, nitems, grid[2], sms;
 };
 
 template <int PART, int X, int Y, int Z, int KIND>

@@ -369,6 +369,7 @@ void *pair_create_plan(const Geom &g, int elem, void *const sets[4], const float
   Plan *pl = new (std::nothrow) Plan();
   if (!pl) return nullptr;
   pl->elem = elem;
+  pl->sms = sm_count();
   pl->geoms.push_back(g);
   pl->plain.assign(1, 1);
   pl->mm.resize(1);
@@ -438,7 +439,7 @@ void launch_stage_pair(const void *plan, const StageArgs &a, int in_set, int *er
   }
   for (int q : {GEN_STR, GEN_VEL, LEAN_BOTH})
     if (pl.grid[q] > 0) entry(pl.elem, kind, q).launch[0](pl, m, a, pl.wk, err, ls[q]);
-  launch_timg(a, side ? side->stream[0] : stream);
+  launch_timg(a, side ? side->stream[0] : stream, pl.sms);
   if (side)
     for (int q = 0; q < SideStream::N; ++q) {
       cudaEventRecord((cudaEvent_t)side->join[q], (cudaStream_t)side->stream[q]);

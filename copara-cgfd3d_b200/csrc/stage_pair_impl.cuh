@@ -1034,7 +1034,10 @@ __device__ __forceinline__ void march(const StageArgs &A, const Maps &M, const W
       if (!compute || warp == 0) return;
       const int d = warp - 1;  // direction
       const int c0 = (PART == PART_VEL) ? 0 : 3;
-      const int cxp = max(cx, 0), cyp = max(cy, 0);  // prefetch boxes start inside the arrays
+      // (a box may lie partly outside its array -- before it at a high-side layer
+      // narrower than the tile, since the low-side layer's cells come first -- and
+      // fetches what lies inside; bx is a multiple of 4 values by xaoff)
+      const int cxp = max(cx, 0), cyp = max(cy, 0);
       const bool on = aux_on[d] &&
                       (d == 0   ? (i0 < g.nabs[0] || i0 + CX > g.ni - g.nabs[1])
                        : d == 1 ? (j0 < g.nabs[2] || j0 + TY > g.nj - g.nabs[3])
@@ -1276,6 +1279,7 @@ struct Plan {
   int elem;                    // storage element type of the field sets
   int zchunk = 0;              // planes of the (first model's) interior z-chunks
   int grid[NLIST];             // CTAs per launch (0: no items)
+  int sms = 0;                 // of the device
   WorkParams params;
   unsigned long long list_id = 0;  // hash of the lists
   int nmodels = 0;             // 0: single-model plan; else a batch of nmodels

@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(128) timg_kernel(StageArgs a) {
 // There the kernel is one chain of loads and arithmetic per thread beside
 // stage kernels that are as short: the 118x95x61 hill 345 us a step with all three
 // components in a thread, 299 with one.  Each component loads the metric
-// again (1.6 times the loads in all), so grids that fill the GPU anyway keep
-// one thread per cell.
+// again (1.6 times the loads in all), so grids of eight blocks per SM of the
+// device (1184 on a B200) or more keep one thread per cell.
 template <typename T>
 __global__ void __launch_bounds__(128) timg_split_kernel(StageArgs a) {
   const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
@@ -176,11 +176,11 @@ void launch_timg_batch(const StageArgs *args, int n, int max_ni, int max_nj, int
 
 namespace {
 template <typename T>
-void timg_t(const StageArgs &a, cudaStream_t s) {
-  constexpr unsigned FULL = 148 * 8;  // blocks that keep every SM's warps busy
+void timg_t(const StageArgs &a, cudaStream_t s, int sms) {
+  const unsigned full = 8u * (unsigned)sms;  // blocks that keep every SM's warps busy
   dim3 block(32, 4, 1);
   dim3 grid((a.g.ni + 31) / 32, (a.g.nj + 3) / 4, 3);
-  if (grid.x * grid.y * 3 < FULL) {
+  if ((size_t)grid.x * grid.y * 3 < full) {
     grid.z = 9;
     timg_split_kernel<T><<<grid, block, 0, s>>>(a);
   } else {
@@ -189,11 +189,11 @@ void timg_t(const StageArgs &a, cudaStream_t s) {
 }
 }  // namespace
 
-void launch_timg(const StageArgs &a, void *stream) {
+void launch_timg(const StageArgs &a, void *stream, int sms) {
   cudaStream_t s = (cudaStream_t)stream;
-  if (a.elem == ELEM_F16) timg_t<__half>(a, s);
-  else if (a.elem == ELEM_BF16) timg_t<__nv_bfloat16>(a, s);
-  else timg_t<float>(a, s);
+  if (a.elem == ELEM_F16) timg_t<__half>(a, s, sms);
+  else if (a.elem == ELEM_BF16) timg_t<__nv_bfloat16>(a, s, sms);
+  else timg_t<float>(a, s, sms);
 }
 
 }  // namespace cgfd

@@ -25,7 +25,8 @@ struct Launch {
   int list;                 // the kernel's (stage_pair_impl.cuh)
   std::vector<int4> items;  // the list it walks
 };
-constexpr int DEVICES = 3, SMS = 148;
+constexpr int DEVICES = 3;
+int sms = 148;
 int device = 0;
 cudaError_t last = cudaSuccess;
 std::map<std::string, std::pair<int, int>> fail;  // call -> calls to pass, then the error
@@ -33,6 +34,7 @@ std::map<const void *, size_t> memory;
 std::set<const void *> fresh;  // allocated (zeros) and not yet written
 std::set<std::pair<int, const void *>> attrs;
 std::vector<Launch> launches;
+std::vector<std::pair<std::string, dim3>> grids;  // of every launch
 std::map<const void *, std::string> names;  // kernels
 dim3 cfg_grid, cfg_block;
 size_t cfg_smem;
@@ -74,11 +76,27 @@ void fake_reset() {
   last = cudaSuccess;
   fail.clear();
   launches.clear();
+  grids.clear();
+  sms = 148;
 }
+void fake_sms(int n) { sms = n; }
 // the call after `pass` more of them fails once with error e
 void fake_fail(const char *call, int pass, int e) { fail[call] = {pass, e}; }
 int fake_blocks() { return (int)memory.size(); }
-void fake_clear_launches() { launches.clear(); }
+void fake_clear_launches() {
+  launches.clear();
+  grids.clear();
+}
+// grid.z of the launches of the kernel so named: all the same, or -1
+int fake_grid_z(const char *kernel) {
+  int z = -1;
+  for (const auto &g : grids)
+    if (g.first.find(kernel) != std::string::npos) {
+      if (z >= 0 && z != (int)g.second.z) return -1;
+      z = (int)g.second.z;
+    }
+  return z;
+}
 // launches of the paired stage kernels so far: list and items
 // (i0, j0, z0, z1, model, part of each)
 int fake_launches() { return (int)launches.size(); }
@@ -123,7 +141,7 @@ cudaError_t cudaGetLastError() {
   return e;
 }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) {
-  *v = SMS;
+  *v = sms;  // (the one attribute the library reads)
   return cudaSuccess;
 }
 cudaError_t cudaMalloc(void **p, size_t n) {
@@ -185,6 +203,7 @@ cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **args, size_t
   if (grid.x == 0 || (smem > 48 * 1024 && !attrs.count({device, f})))
     return ret(cudaErrorInvalidValue);
   const std::string &n = names[f];
+  grids.push_back({n, grid});
   if (n.find("pair_kernel") != std::string::npos) {
     // template arguments <T, X, Y, Z, KIND, batched, LIST>
     const int list = n[n.find("ELi", n.find("Lb")) + 3] - '0';

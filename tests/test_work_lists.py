@@ -188,3 +188,18 @@ def test_autotuner_times_a_list_once(fake, grid, lists):
     timed, chosen = shapes[:-1], shapes[-1]
     assert len(timed) == len(set(timed)) >= lists and chosen in timed
     s.close()
+
+
+@pytest.mark.parametrize("kernel", [cgfd.KERNEL_FUSED, cgfd.KERNEL_SCALAR])
+@pytest.mark.parametrize("sms,split", [(148, True), (16, False)])
+def test_traction_image_is_split_where_it_does_not_fill_the_device(fake, kernel, sms, split):
+    """A thread per component below eight blocks per SM of the device in use:
+    3 * 24 * 3 blocks of this grid."""
+    fake.fake_sms(sms)
+    m = _model(ni=96, nj=96)
+    s = cgfd.Solver(m.desc(kernel=kernel))
+    m.load(s)
+    s.prepare()
+    assert fake.fake_grid_z(b"timg_split_kernel") == (9 if split else -1)
+    assert fake.fake_grid_z(b"timg_kernel") == (-1 if split else 3)
+    s.close()
