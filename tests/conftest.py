@@ -1,7 +1,9 @@
 """Test configuration: markers and import paths.
 
-`-m gpu` tests need a B200 and the built libraries (libcgfd.so, and the
-reference parity driver oracle/_ref/ref_wavesim); `-m "not gpu"` tests run on
+`-m gpu` tests need a B200 and the built library libcgfd.so; those against the
+reference's own runtime also its driver oracle/_ref/ref_wavesim, built from the
+reference's sources (oracle/ref/Makefile), and are skipped without it;
+`-m "not gpu"` tests run on
 the CPU: the oracle against the reference's golden vectors, the host-side
 pre-processing, and the C ABI's symbol table.
 """
@@ -15,6 +17,18 @@ for p in (os.path.join(ROOT, "copara-cgfd3d_b200", "python"), os.path.join(ROOT,
           os.path.join(ROOT, "tests"), os.path.join(ROOT, "tests", "golden")):
     if p not in sys.path:
         sys.path.insert(0, p)
+
+
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_call(item):
+    """Tests that ask for the reference's driver (refio.run raises
+    FileNotFoundError without it) are skipped where it was not built."""
+    outcome = yield
+    if outcome.excinfo is None or not issubclass(outcome.excinfo[0], FileNotFoundError):
+        return
+    import refio
+    if not refio.available() and "ref_wavesim" in str(outcome.excinfo[1]):
+        outcome.force_exception(pytest.skip.Exception(str(outcome.excinfo[1])))
 
 
 def pytest_configure(config):

@@ -3,11 +3,18 @@ grid; general: the rest) at the edges of their tiles: grids whose layers end
 on, before and after tile boundaries (32 cells in x, 8 in y), with and without
 a bottom layer of its own z-chunk, and with a few interior planes only.
 
+Which items each grid has is checked on the CPU (test_work_lists.py).
+
 FP32 storage against the FP64 oracle within the parity bound of the other
 tests, 1e-5 relative L2.  16-bit storage against FP32 storage: a store rounds
-by at most 2^-11 (FP16) or 2^-8 (BF16) of the value and a step stores each
+by at most u = 2^-11 (FP16) or 2^-8 (BF16) of the value and a step stores each
 field five times (W three times, the accumulator, FW), so three steps differ
-by at most 15 of those."""
+by at most 15 of those.  Four steps, which run each of the four stencil
+patterns, alone and in a batch (whose kernels are compilations of their own), are
+compared on every plane of cells along each axis by itself, so that an error
+confined to one edge shows: there the 20 roundings of a field and those it takes
+over from the others are independent, sqrt(20) u in the root mean square, held to
+twice that; FP32 to 1e-5."""
 import numpy as np
 import pytest
 
@@ -68,3 +75,106 @@ def test_item_lists_match_the_oracle(grid):
         w = _run(m, init, store)
         for c in range(9):
             assert rel_l2(w[c], got[c]) < 15 * ulp, (store, cgfd.COMPONENTS[c])
+
+
+def _fields(s):
+    return np.stack([s.get_field(c) for c in range(9)])
+
+
+def _start(s, m, init, storage):
+    m.load(s)
+    if storage == cgfd.STORE_F16:
+        s.set_field_scales([0] * 3 + [14] * 6)
+    for c in range(9):
+        s.set_field(c, init[c])
+
+
+def _oracle4(m, init):
+    o = pyoracle.OracleSolver(m.desc(), 0)
+    m.load(o)
+    for c in range(9):
+        o.set_field(c, init[c])
+    o.step(4)
+    ref = np.stack([o.get_field(c, 0) for c in range(9)])
+    o.close()
+    return ref
+
+
+def _plane_errors(got, ref):
+    """Largest error of a plane of cells along x, y or z, over its values' norm
+    (at least a tenth of the component's mean plane and 1% of the largest
+    component of the group, as comp_errors)."""
+    d, r = (np.asarray(a, np.float64)[:, 3:-3, 3:-3, 3:-3] for a in (got - ref, ref))
+    group = [np.sqrt((r[:3] ** 2).sum((1, 2, 3)).max()), np.sqrt((r[3:] ** 2).sum((1, 2, 3)).max())]
+    worst = 0.0
+    for c in range(9):
+        total = max(np.sqrt((r[c] ** 2).sum()), 1e-2 * group[c >= 3])
+        for ax in range(3):
+            other = tuple(a for a in range(3) if a != ax)
+            n = np.sqrt((r[c] ** 2).sum(other))
+            n = np.maximum(n, 0.1 * total / np.sqrt(r.shape[1 + ax]))
+            worst = max(worst, (np.sqrt((d[c] ** 2).sum(other)) / n).max())
+    return worst
+
+
+BOUND = {cgfd.STORE_F32: 1e-5, cgfd.STORE_F16: 2 * 20 ** 0.5 * 2.0 ** -11,
+         cgfd.STORE_BF16: 2 * 20 ** 0.5 * 2.0 ** -8}
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+def test_every_stencil_pattern_plane_by_plane(grid):
+    m = _model(grid)
+    init = cases.random_fields(m, 23)
+    ref = _oracle4(m, init)
+    for storage, bound in BOUND.items():
+        s = cgfd.Solver(m.desc(storage=storage))
+        _start(s, m, init, storage)
+        s.step(4)
+        e = _plane_errors(_fields(s), ref)
+        s.close()
+        assert e < bound, (storage, e)
+
+
+@pytest.mark.parametrize("storage", list(BOUND), ids=["f32", "f16", "bf16"])
+def test_every_stencil_pattern_in_a_batch_plane_by_plane(storage):
+    ms = [_model(g) for g in GRIDS]
+    b = cgfd.Batch([m.desc(storage=storage) for m in ms])
+    inits = [cases.random_fields(m, 30 + k) for k, m in enumerate(ms)]
+    for m, s, init in zip(ms, b.models, inits):
+        _start(s, m, init, storage)
+    b.step(4)
+    for m, s, init in zip(ms, b.models, inits):
+        e = _plane_errors(_fields(s), _oracle4(m, init))
+        assert e < BOUND[storage], ((m.ni, m.nj, m.nk), e)
+    b.close()
+
+
+@pytest.mark.parametrize("axis,at", [(0, 40), (1, 20), (2, 15)])
+def test_profiles_that_are_not_one_off_the_layers(axis, at):
+    """B other than 1 in the interior: such a model has general items only, alone
+    and beside a plain one in a batch (the lists are rebuilt when the profiles are
+    known, and once more when plain ones replace them)."""
+    plain, m = _model(GRIDS[0]), _model(GRIDS[0])
+    m.pml[1][axis][3 + at:3 + at + 2] = 1.25
+    init = cases.random_fields(m, 41)
+    ref, ref_plain = _oracle4(m, init), _oracle4(plain, init)
+    assert _plane_errors(ref, ref_plain) > 1e-2
+    s = cgfd.Solver(m.desc())
+    _start(s, m, init, cgfd.STORE_F32)
+    s.step(4)
+    assert _plane_errors(_fields(s), ref) < 1e-5
+    s.close()
+    b = cgfd.Batch([plain.desc(), m.desc()])
+    for mm, s in zip((plain, m), b.models):
+        _start(s, mm, init, cgfd.STORE_F32)
+    b.step(4)
+    assert _plane_errors(_fields(b.models[0]), ref_plain) < 1e-5
+    assert _plane_errors(_fields(b.models[1]), ref) < 1e-5
+    b.close()
+    s = cgfd.Solver(m.desc())
+    _start(s, m, init, cgfd.STORE_F32)
+    s.prepare()
+    s.upload_pml(*plain.pml)
+    s.step(4)
+    assert _plane_errors(_fields(s), ref_plain) < 1e-5
+    s.close()

@@ -99,9 +99,10 @@ def test_kernel_attributes_are_set_on_every_device(fake, kernel, storage):
 
 
 TILE_X, TILE_Y, LFD = 32, 8, 3
-GRIDS = [  # ni, nj, nk, nabs
+GRIDS = [  # ni, nj, nk, nabs (the first six are those of test_gpu_lean_tiles.py)
     (96, 40, 24, (8, 8, 8, 8, 8, 0)),
     (64, 16, 12, (0, 0, 0, 0, 0, 0)),
+    (65, 17, 11, (0, 0, 0, 0, 3, 0)),
     (101, 27, 19, (32, 5, 3, 1, 4, 0)),
     (100, 9, 20, (1, 35, 0, 0, 9, 0)),
     (40, 30, 13, (4, 4, 4, 4, 6, 0)),
@@ -123,7 +124,7 @@ def _covered(it, model):
 
 
 @pytest.mark.parametrize("plain", [True, False], ids=["plain", "not_plain"])
-@pytest.mark.parametrize("grids", [[g] for g in GRIDS] + [GRIDS[:5]],
+@pytest.mark.parametrize("grids", [[g] for g in GRIDS] + [GRIDS[:6]],
                          ids=["x".join(map(str, g[:3])) for g in GRIDS] + ["batch"])
 def test_items_cover_every_cell_once(fake, grids, plain):
     """Every cell is an item's of each part exactly once; lean items hold cells
