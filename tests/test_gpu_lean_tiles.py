@@ -15,6 +15,8 @@ compared on every plane of cells along each axis by itself, so that an error
 confined to one edge shows: there the 20 roundings of a field and those it takes
 over from the others are independent, sqrt(20) u in the root mean square, held to
 twice that; FP32 to 1e-5."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -178,3 +180,29 @@ def test_profiles_that_are_not_one_off_the_layers(axis, at):
     s.step(4)
     assert _plane_errors(_fields(s), ref_plain) < 1e-5
     s.close()
+
+
+@pytest.mark.parametrize("storage", list(BOUND), ids=["f32", "f16", "bf16"])
+@pytest.mark.parametrize("grid", [GRIDS[0], GRIDS[3]])
+def test_every_direction_in_every_stage(grid, storage):
+    """The four stages of a step in each of the eight stencil directions, driven
+    one by one: with the batched patterns above these are the kernels of every
+    direction, stage kind, item list and storage type.  (A step's five roundings
+    of each field, within the bound for four steps.)"""
+    m = _model(grid)
+    init = cases.random_fields(m, 51)
+    s, o = cgfd.Solver(m.desc(storage=storage)), pyoracle.OracleSolver(m.desc(), 0)
+    _start(s, m, init, storage)
+    m.load(o)
+    for d in itertools.product((1, -1), repeat=3):
+        for c in range(9):  # (the layers' auxiliaries go on)
+            s.set_field(c, init[c])
+            o.set_field(c, init[c])
+        for rk in range(4):
+            s.rk_stage(rk, 0, *d)
+            o.rk_stage(rk, 0, *d)
+        ref = np.stack([o.get_field(c, 0) for c in range(9)])
+        e = _plane_errors(_fields(s), ref)
+        assert e < BOUND[storage], (d, e)
+    s.close()
+    o.close()
