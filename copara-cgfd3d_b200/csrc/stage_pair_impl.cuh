@@ -16,8 +16,9 @@
 // where the one kernel for both kept two (three), and runs both parts of a
 // tile side by side (they share the stage input's V and sigma in L2).  The
 // march is bound by latency and instruction fetch before it is bound by HBM,
-// so resident warps count: the 400x400x200 hill's lean launch at three CTAs
-// moves 66-69% of the DRAM peak (52-58% before).  Unrolling the march by 2 or
+// so resident warps count: at three CTAs the lean launch of the 256x256x128
+// hill's inner stage moves 67% of the DRAM peak (52-58% before), that of the
+// 600x600x250 one 5.8 TB/s.  Unrolling the march by 2 or
 // 5 (no register moves in the z-window) is slower: 14.9 -> 15.2 and 16.5 ms on
 // the 600x600x250 hill; four CTAs with two slots too (15.4 ms).
 //

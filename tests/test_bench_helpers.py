@@ -38,6 +38,18 @@ def test_curved_metric_adds_its_coefficients():
     assert b - 144 * 4 * (m.cells + pairs) > flat_like
 
 
+def test_least_bytes_keep_the_coefficients():
+    """117 of 144 state values, 78 of 144 auxiliary values, the same media and
+    metric."""
+    bench = _bench()
+    for m in (models.small_flat(nt=4), models.small_hill(nt=4)):
+        pairs = ((m.nabs[0] + m.nabs[1]) * m.nj * m.nk + (m.nabs[2] + m.nabs[3]) * m.ni * m.nk +
+                 (m.nabs[4] + m.nabs[5]) * m.ni * m.nj)
+        for elem in (4, 2):
+            assert (bench.algorithmic_bytes_per_step(m, elem) - bench.least_bytes_per_step(m, elem)
+                    == 27 * elem * m.cells + 66 * 4 * pairs)
+
+
 def test_workload_names_and_traffic_lookup():
     bench = _bench()
     assert bench.workload_name("hill600") == "gaussian_hill_600x600x250_random_layers_pml20"

@@ -1,8 +1,8 @@
 """The bounded device waits of the stage kernels (failure detection without a
 GPU fault).  Every mbarrier wait of the default kernel gives up after a
 limit; cgfd_test_withhold_copy shortens the limit to a few milliseconds and
-makes the velocity part's first CTA withhold one tensor copy, so that its
-wait for that plane runs out: nothing faults or hangs, the CTA records the
+makes the CTA with a list's first velocity item withhold one tensor copy, so that
+its wait for that plane runs out: nothing faults or hangs, the CTA records the
 expiry, drains its own copies (bounded) and returns, and cgfd_sync reports
 CGFD_ERR_TIMEOUT.  A new solver on the same device then runs normally (its
 seismograms equal the FP64 oracle's)."""
