@@ -210,7 +210,7 @@ def algorithmic_bytes_per_step(m, elem=4):
 
 
 def least_bytes_per_step(m, elem=4):
-    """The floor that the design notes use: 117 state values per cell (18+27+27+45:
+    """The least a step can move: 117 state values per cell (18+27+27+45:
     every stage reads its input and FW once and writes its result once, the last
     one combines the three results; the kernels keep an accumulator instead, 126),
     and the same share for six auxiliaries per pair."""

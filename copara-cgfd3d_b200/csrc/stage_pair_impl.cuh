@@ -596,7 +596,8 @@ __device__ __forceinline__ void vel_pair(const StageArgs &a, const Pair &e, cons
   f2 hw[3], hax[3], hay[3], haz[3];
   // 16-bit storage: the order of rounding of Geom::kx0 (such a pair has no
   // auxiliaries and B = 1); rows of the range that fill no tile, and models too
-  // shallow for lean items, come through here
+  // shallow for lean items, come through here.  Both orders are computed: 0.3-0.6%
+  // of a 16-bit step (256x256x128 FP16 30.06 -> 30.22 ms a pass), a branch 1.6-2.8%.
   const bool kept = sizeof(T) != 4 && e.kept && !pl.zpml;
 #pragma unroll
   for (int q = 0; q < 3; ++q) {

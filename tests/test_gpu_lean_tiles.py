@@ -15,6 +15,7 @@ compared on every plane of cells along each axis by itself, so that an error
 confined to one edge shows: there the 20 roundings of a field and those it takes
 over from the others are independent, sqrt(20) u in the root mean square, held to
 twice that; FP32 to 1e-5."""
+import ctypes as C
 import itertools
 
 import numpy as np
@@ -206,3 +207,36 @@ def test_every_direction_in_every_stage(grid, storage):
         assert e < BOUND[storage], (d, e)
     s.close()
     o.close()
+
+
+def test_planes_past_2_to_the_15():
+    """A grid of 33000 planes (z ranges that once overflowed an item's two 16-bit
+    halves), both item lists, against the untiled kernel on the same inputs:
+    FP32 roundings of one step, 1e-5."""
+    ni, nj, nk, nabs = 32, 10, 33000, (0, 0, 1, 1, 8, 0)
+    shape = (ni + 6, nj + 6, nk + 6)
+    rng = np.random.default_rng(61)
+    prof = [[np.full(n, v) for n in shape] for v in (0.0, 1.0, 0.0)]  # APD, B, DB
+    for ax, cells in ((1, [3, nj + 2]), (2, list(range(3, 11)))):
+        for p, v in zip(prof, (2.0, 1.5, 20.0)):
+            p[ax][cells] = v
+    # a random block, repeated in z with another amplitude each time
+    block = rng.standard_normal((9, ni, nj, 100)).astype(np.float32)
+    amp = np.repeat(rng.uniform(0.5, 2.0, nk // 100).astype(np.float32), 100)
+    out = []
+    for kernel in (cgfd.KERNEL_FUSED, cgfd.KERNEL_SIMPLE):
+        s = cgfd.Solver(cgfd.Desc(ni=ni, nj=nj, nk=nk, steph=100.0, stept=0.005, nt=2,
+                                  con_index=nk // 2, hybrid_grid=1,
+                                  nabs=(C.c_int * 6)(*nabs), kernel=kernel))
+        zero, one = np.zeros(shape), np.ones(shape)
+        s.upload_metric(zero, zero, one, one)
+        s.upload_media(*(np.full(shape, v, np.float32) for v in (6000.0, 3464.0, 2670.0)))
+        s.upload_pml(*prof)
+        for c in range(9):
+            f = np.zeros(shape, np.float32)
+            f[3:-3, 3:-3, 3:-3] = np.tile(block[c], nk // 100) * amp * (1.0 if c < 3 else 1e7)
+            s.set_field(c, f)
+        s.step(1)
+        out.append(_fields(s))
+        s.close()
+    assert _plane_errors(*out) < 1e-5
