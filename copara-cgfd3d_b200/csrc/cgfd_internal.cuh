@@ -233,8 +233,8 @@ struct SideStream {
 void launch_stage_pair(const void *plan, const StageArgs &a, int in_set, int *err, void *stream,
                        const SideStream *side = nullptr);
 int pair_plan_info(const void *plan, int *zchunk, int *grid_general, int *grid_lean);
-// A batch of models (one storage type) in one persistent launch per stage
-// part: per-model buffers as n x 4 sets, n media, n metrics, n x 3
+// A batch of models (one storage type) in one persistent launch per part and
+// item list of a stage: per-model buffers as n x 4 sets, n media, n metrics, n x 3
 // auxiliaries.
 void *pair_create_batch_plan(int n, const Geom *gs, void *const *sets, const float *const *media,
                              const float *const *metric, float *const *aux, int elem);

@@ -2165,7 +2165,7 @@ struct cgfd_batch {
   int max_foc = 0;  // most focal points of any member
   int max_sp = 0;   // longest spread list (smoothed sources) of any member
   cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
-  // launch shape: false, one persistent launch per stage part over every
+  // launch shape: false, persistent launches (per part and item list) over every
   // member's items (uneven, small members share the GPU without tails);
   // true, every member's own step graphs on its own stream (members large
   // enough to fill the GPU alone run the single-model kernels, whose stage

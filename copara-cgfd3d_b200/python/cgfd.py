@@ -437,8 +437,8 @@ def mlp_gradient(weights, x, t):
 
 
 class Batch:
-    """Several models stepped together in one persistent launch per stage
-    part (cgfd_batch_*); models[i] is the member Solver for uploads, fields
+    """Several models stepped together in persistent launches over all their
+    work items (cgfd_batch_*); models[i] is the member Solver for uploads, fields
     and seismograms."""
 
     def __init__(self, descs):

@@ -344,7 +344,7 @@ int cgfd_test_withhold_copy(cgfd_solver *h, double wait_limit_s, int withhold);
 /* A batch steps n independent models (each its own grid, medium, PML,
  * sources, receivers, dt and learned layer; one storage type for all, default
  * kernel family) together.  Launch shape CGFD_BATCH_PERSISTENT (the default):
- * one persistent launch per stage part over every member's work items, so
+ * persistent launches over every member's work items in every stage, so
  * that uneven, small models share the GPU without per-model launch tails.
  * CGFD_BATCH_MEMBERS: every member's own step graphs, each member on its own
  * stream (members that fill the GPU alone run at the single-model kernels'

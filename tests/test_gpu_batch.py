@@ -1,7 +1,7 @@
 """Batched models and the work-list autotuner.
 
-A batch steps several independent models through one persistent launch per
-stage part; its per-cell arithmetic is the single-model kernel's source, so
+A batch steps several independent models through persistent launches over all
+their work items; its per-cell arithmetic is the single-model kernel's source, so
 every member's seismograms and fields must equal those of the same model run
 alone up to FP32 rounding (the batched instantiation is a separate
 compilation; measured <= 9.3e-7 relative L2 per component over 24 steps, held
